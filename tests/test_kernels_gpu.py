@@ -342,6 +342,16 @@ def test_sampler_distribution_and_modes():
     assert bool((tok == logits[0].bfloat16().float().argmax()).all())
 
 
+def test_sampler_never_takes_a_token_of_no_weight():
+    """A uniform draw that rounds up to one must not become infinite noise: 4000 rows of 152 064 tokens hold about 36 such draws."""
+    from verl_b200 import ops
+
+    logits = torch.zeros(1, 152064, device="cuda")
+    logits[0, 77] = 100.0
+    tok, _ = ops.sample(logits.expand(4000, -1), seed=11, step=torch.zeros(1, device="cuda", dtype=torch.long))
+    assert bool((tok == 77).all())
+
+
 @pytest.mark.parametrize("B,Hq,Hk,D,bs,maxlen", [(5, 28, 4, 128, 16, 700), (3, 4, 2, 64, 16, 300), (2, 32, 4, 128, 32, 3000),
                                                  (4, 40, 8, 128, 16, 150), (3, 32, 2, 128, 128, 1000),
                                                  (2, 8, 8, 128, 8, 260),

@@ -183,6 +183,9 @@ __device__ __forceinline__ uint4 philox(uint4 c, uint2 k) {
   return c;
 }
 __device__ __forceinline__ float u01(uint32_t x) { return ((float)(x >> 8) + 0.5f) * (1.f / 16777216.f); }
+// Gumbel noise of a uniform draw. The largest draws round up to one (16777215.5 has no fp32 form) and the fast logarithm is off by
+// up to 2^-22 there: without the floor -log(u) could be zero, the noise infinite, and one token in 2^24 a draw no matter its logit.
+__device__ __forceinline__ float gumbel(uint32_t x) { return -__logf(fmaxf(-__logf(u01(x)), 2.98e-8f)); }
 
 // Four consecutive logits starting at v0 (a multiple of 4) as floats; elements past V read as -inf. `vec` says that the
 // row base is aligned for one 16-byte (fp32) / 8-byte (bf16) load.
@@ -241,7 +244,7 @@ __device__ __forceinline__ void sample_row_one_pass(const T* __restrict__ lg, in
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (v0 + j < V) {
-        const float sc = greedy ? x[j] : x[j] - __logf(-__logf(u01(rr[j])));
+        const float sc = greedy ? x[j] : x[j] + gumbel(rr[j]);
         if (sc > best) {  // indices only grow inside a thread: ties keep the lowest
           best = sc;
           best_i = v0 + j;
@@ -394,7 +397,7 @@ __global__ void sample_kernel(const T* __restrict__ logits, long long row_stride
         const float e = __expf(x);
         if (e / z >= thr) {
           zr += e;
-          const float g = greedy ? 0.f : -__logf(-__logf(u01(rr[j])));
+          const float g = greedy ? 0.f : gumbel(rr[j]);
           const float s = x + g;
           if (s > best) {
             best = s;
