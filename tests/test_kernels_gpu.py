@@ -342,6 +342,35 @@ def test_sampler_distribution_and_modes():
     assert bool((tok == logits[0].bfloat16().float().argmax()).all())
 
 
+@pytest.mark.parametrize("V", [7, 1023, 1025, 4099, 32771, 152064])  # one block, the guesses' limit, a ragged last group, clusters
+@pytest.mark.parametrize("B", [1, 3, 75, 150])                      # 8, 4, 1 blocks per row and more rows than SMs
+@pytest.mark.parametrize("k,p", [(-1, 0.9), (5, 1.0), (12, 0.8), (3, 0.99)])
+def test_sampler_support_and_logprob(V, B, k, p):
+    """Tokens come from the smaller of the top-k set and the nucleus; log-probs are those of the renormalised support. The strong
+    tokens are 0.3 apart (so no set hangs on rounding), the tail together weighs less than a thousandth of the last of them."""
+    from verl_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(V + B)
+    n = min(V, 40)
+    logits = torch.full((B, V), -40.0, device="cuda")
+    where = torch.stack([torch.randperm(V, device="cuda", generator=g)[:n] for _ in range(B)])
+    logits.scatter_(1, where, -0.3 * torch.arange(n, device="cuda").repeat(B, 1))
+    step = torch.zeros(1, dtype=torch.long, device="cuda")
+    tok, lp = ops.sample(logits, top_k=torch.full((B,), k, dtype=torch.int32, device="cuda"), top_p=torch.full((B,), p, device="cuda"),
+                         seed=3, step=step)
+    d = torch.softmax(logits[0].double(), -1).sort(descending=True).values
+    size = V
+    if 0 < k < V:
+        size = k
+    if p < 1:
+        size = min(size, int((d.cumsum(0) < p).sum()) + 1)
+    keep = where[:, :size]
+    hit = keep == tok[:, None]
+    assert bool(hit.any(1).all())
+    ref = torch.log_softmax(-0.3 * torch.arange(size, device="cuda", dtype=torch.float64), -1)[hit.float().argmax(1)]
+    assert float((lp - ref).abs().max()) < 2e-5  # fast exp, log and fp32 sums of up to 40 terms
+
+
 def test_sampler_never_takes_a_token_of_no_weight():
     """A uniform draw that rounds up to one must not become infinite noise: 4000 rows of 152 064 tokens hold about 36 such draws."""
     from verl_b200 import ops
