@@ -53,3 +53,25 @@ def test_out_of_memory_in_a_training_forward_falls_back_to_recomputation(monkeyp
     monkeypatch.setattr(zmod._UnitFnKeep, "forward", real)
     assert calls["n"] == 1 and eng._keep_cap == 0 and eng._layers_to_keep(20) == 0
     torch.testing.assert_close(got, ref)
+
+
+def test_second_backward_recomputes_a_kept_unit():
+    """``retain_graph``: the kept graph of a unit serves one backward, a further one recomputes the unit and adds the same gradient."""
+    import torch
+
+    from verl_b200.models import preset
+    from verl_b200.models.transformer import PackedBatch
+    from verl_b200.workers.engine.native import NativeEngine
+
+    cfg = preset("tiny-qwen2", tie_word_embeddings=False)
+    ids = torch.randint(3, cfg.vocab_size, (20,), generator=torch.Generator().manual_seed(0))
+    batch = PackedBatch(ids, torch.arange(20), torch.tensor([0, 20], dtype=torch.int32), 20)
+    eng = NativeEngine(cfg, {"keep_activation_layers": cfg.num_hidden_layers}, {"lr": 1e-3}, device="cpu", seed=1).initialize()
+    with eng.train_mode():
+        eng.optimizer_zero_grad()
+        lp, ent = eng.forward_logprob(batch, torch.arange(19), ids[1:], 1.0)
+        loss = (ent - lp).mean()
+        loss.backward(retain_graph=True)
+        once = eng.zero.grad.clone()
+        loss.backward()
+    torch.testing.assert_close(eng.zero.grad, 2 * once)

@@ -402,30 +402,37 @@ class _UnitFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, *grads):
-        zero, unit = ctx.zero, ctx.unit
-        inputs = [t.detach().requires_grad_(t.is_floating_point()) for t in ctx.saved_tensors]
-        zero.gather(unit, for_backward=True)
-        try:
-            with torch.enable_grad():
-                outs = ctx.fn(*_expand(ctx.mask, inputs))
-            outs = (outs,) if ctx.single else outs
-            pairs = [(o, g) for o, g in zip(outs, grads) if g is not None and isinstance(o, torch.Tensor) and o.requires_grad]
-            if pairs:
-                torch.autograd.backward([o for o, _ in pairs], [g for _, g in pairs])
-            zero.reduce_grads(unit)
-        finally:
-            zero.release(unit)
-        return (None, None, None, None) + tuple(t.grad if t.requires_grad else None for t in inputs) + (None,)
+        return _recompute_backward(ctx, grads)
+
+
+def _recompute_backward(ctx, grads):
+    """Gather again, recompute the unit from the saved inputs with autograd, back-propagate."""
+    zero, unit = ctx.zero, ctx.unit
+    inputs = [t.detach().requires_grad_(t.is_floating_point()) for t in ctx.saved_tensors]
+    zero.gather(unit, for_backward=True)
+    try:
+        with torch.enable_grad():
+            outs = ctx.fn(*_expand(ctx.mask, inputs))
+        outs = (outs,) if ctx.single else outs
+        pairs = [(o, g) for o, g in zip(outs, grads) if g is not None and isinstance(o, torch.Tensor) and o.requires_grad]
+        if pairs:
+            torch.autograd.backward([o for o, _ in pairs], [g for _, g in pairs])
+        zero.reduce_grads(unit)
+    finally:
+        zero.release(unit)
+    return (None, None, None, None) + tuple(t.grad if t.requires_grad else None for t in inputs) + (None,)
 
 
 class _UnitFnKeep(torch.autograd.Function):
     """Like :class:`_UnitFn` but the unit's activations are kept: the forward records the unit's autograd graph and
     the backward runs it (no recomputation) after gathering the parameters again. The graph refers to the unit's
-    ``Parameter`` objects, whose storage is re-bound by every gather, so it reads the re-gathered weights."""
+    ``Parameter`` objects, whose storage is re-bound by every gather, so it reads the re-gathered weights. It is gone after
+    that: a further backward (``retain_graph``) recomputes the unit."""
 
     @staticmethod
     def forward(ctx, zero: ZeroShardedParams, unit: ZeroUnit, fn: Callable, mask: tuple, *tensors):
-        ctx.zero, ctx.unit = zero, unit
+        ctx.zero, ctx.unit, ctx.fn, ctx.mask = zero, unit, fn, mask
+        ctx.save_for_backward(*tensors[:-1])
         inputs = [t.detach().requires_grad_(t.is_floating_point()) for t in tensors[:-1]]
         zero.gather(unit)
         try:
@@ -440,6 +447,8 @@ class _UnitFnKeep(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, *grads):
+        if ctx.outs is None:
+            return _recompute_backward(ctx, grads)
         zero, unit = ctx.zero, ctx.unit
         inputs, outs = ctx.inputs, ctx.outs
         ctx.inputs = ctx.outs = None

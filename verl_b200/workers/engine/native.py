@@ -692,7 +692,11 @@ class NativeEngine(BaseEngine):
                     spp.append((p * p).sum(-1))
             return (*out, torch.cat(spp) if spp else x.new_zeros(0, dtype=torch.float32))
 
-        out = self._sp_merge(unit_call(z, self._head_unit, head, hidden, residual))
+        # The head keeps its activations: final-norm rows [N, H] and two numbers per row, where recomputing it would repeat its
+        # product with the whole vocabulary (6.8 of 70 ms of an update on 4 layers of the 7B widths). Recomputed all the same
+        # under pipeline parallelism (many micro-batches wait for their backward) and after an out-of-memory error.
+        out = self._sp_merge(unit_call(z, self._head_unit, head, hidden, residual,
+                                       keep_activations=self.pp_size == 1 and self._keep_cap != 0))
         return self._pp_share(out, None, rows.numel()) if self.pp_size > 1 else out
 
     def forward_values(self, batch: PackedBatch, rows: torch.Tensor):
