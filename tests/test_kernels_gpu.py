@@ -557,6 +557,69 @@ def test_moe_grouped_gemm_matches_expert_loop():
     close(g2.main_grad - 1.0, gr.grad, 3e-2)
 
 
+@pytest.mark.parametrize("T,E,k,H,I,first,total", [
+    (1, 8, 2, 128, 64, 0, 8),        # fewer pairs than experts
+    (24, 128, 8, 256, 64, 0, 128),   # a decode step
+    (129, 3, 1, 64, 128, 0, 3),      # shares just above one block of rows
+    (700, 16, 4, 192, 64, 4, 32),    # experts 4 .. 19 of 32 (a replica's part): other pairs have no row
+    (5000, 2, 1, 64, 64, 0, 2),      # several chunks of pairs per expert
+])
+def test_routed_mlp_forms(T, E, k, H, I, first, total):
+    """Places, padding rows, weighted sum and all gradients of the routed MLP against an fp64 loop over the experts, and a buffer
+    full of NaN behind every allocation it makes (nothing undefined may reach a result)."""
+    from verl_b200 import ops
+    from verl_b200.ops.moe import moe_mlp
+
+    gen = torch.Generator(device="cuda").manual_seed(T + E)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    x = rnd(T, H).bfloat16().requires_grad_(True)
+    gate_up, down = ((rnd(*s) * 0.1).bfloat16().requires_grad_(True) for s in ((E, 2 * I, H), (E, H, I)))
+    top_i = rnd(T, total).topk(k, -1).indices
+    top_w = torch.rand(T, k, device="cuda", generator=gen).requires_grad_(True)
+    dy = rnd(T, H).bfloat16()
+    for n in (T * k * H, (T * k + E * 127) * H, (T * k + E * 127) * 2 * I, T * H):  # freed at once: found again by the next allocations
+        torch.full((n,), float("nan"), dtype=torch.bfloat16, device="cuda")
+    y = moe_mlp(x, top_i, top_w, gate_up, down, ops.swiglu, expert_offset=first, num_experts=total)
+    y.backward(dy)
+    xr, wr, gr, dr = (t.detach().double().requires_grad_(True) for t in (x, top_w, gate_up, down))
+    ref = torch.zeros(T, H, dtype=torch.float64, device="cuda")
+    for e in range(E):
+        t, j = (top_i == first + e).nonzero(as_tuple=True)
+        gu = xr[t] @ gr[e].t()
+        h = torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]
+        ref = ref.index_add(0, t, (h @ dr[e].t()) * wr[t, j][:, None])
+    ref.backward(dy.double())
+    # three bf16 roundings on the way forward and six back, 2^-9 each, against the largest value
+    for got, want, roundings in ((y, ref, 3), (x.grad, xr.grad, 6), (top_w.grad, wr.grad, 6), (gate_up.grad, gr.grad, 6),
+                                 (down.grad, dr.grad, 6)):
+        want = want.detach()
+        err = float((got.detach().double() - want).abs().max())
+        assert err <= roundings * 2.0 ** -8 * float(want.abs().max()) + 1e-12, (got.shape, err, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("E,k", [(8, 2), (33, 8), (128, 8), (300, 32)])
+@pytest.mark.parametrize("renorm", [True, False])
+@pytest.mark.parametrize("given", [False, True])
+def test_moe_gate_matches_softmax_topk(E, k, renorm, given):
+    """Experts (ties included: bf16 logits repeat), weights and gradient of the gate against torch in fp64."""
+    from verl_b200.ops.moe import moe_gate
+
+    gen = torch.Generator(device="cuda").manual_seed(E)
+    z = torch.randn(37, E, device="cuda", generator=gen).bfloat16().requires_grad_(True)
+    fixed = torch.rand(37, E, device="cuda", generator=gen).topk(k, -1).indices if given else None
+    w, idx = moe_gate(z, k, renorm, fixed)
+    g = torch.randn(37, k, device="cuda", generator=gen)
+    w.backward(g)
+    zr = z.detach().double().requires_grad_(True)
+    want = fixed if given else torch.sort(zr.detach(), dim=-1, descending=True, stable=True).indices[:, :k]
+    assert torch.equal(idx, want)
+    p = torch.softmax(zr, -1).gather(1, want)
+    p = p / p.sum(-1, keepdim=True) if renorm else p
+    p.backward(g.double())
+    assert float((w.double() - p).abs().max()) < 1e-6
+    assert float((z.grad.double() - zr.grad).abs().max()) <= 2.0 ** -8 * float(zr.grad.abs().max()) + 1e-9
+
+
 def test_bounded_device_wait_reports_status_and_context_survives():
     """A cross-rank barrier whose peer never arrives: the kernel gives up after its time limit, records the wait in
     the status word and returns; the host reads the code and the context keeps working."""

@@ -198,8 +198,9 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __rest
 
 // ------------------------------- SwiGLU --------------------------------------
 // gu: [T, 2I] (gate | up), out: [T, I]
+// blk_expert (null: none): rows of a buffer sorted by expert, blocks of 128 rows without one are left out.
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T,
-                                  int I) {
+                                  int I, const int* __restrict__ blk_expert) {
   pdl_trigger();
   pdl_wait();
   const int nvec = I >> 3;
@@ -208,6 +209,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
        idx += (long long)gridDim.x * blockDim.x) {
     const long long t = idx / nvec;
     const int v = idx % nvec;
+    if (blk_expert != nullptr && blk_expert[t >> 7] < 0) continue;
     float g[8], u[8], o[8];
     load8(gu + t * 2 * I + v * 8, g);
     load8(gu + t * 2 * I + I + v * 8, u);
@@ -218,13 +220,15 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
 }
 
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dout,
-                                  __nv_bfloat16* __restrict__ dgu, long long T, int I) {
+                                  __nv_bfloat16* __restrict__ dgu, long long T, int I,
+                                  const int* __restrict__ blk_expert) {
   const int nvec = I >> 3;
   const long long total = T * nvec;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     const long long t = idx / nvec;
     const int v = idx % nvec;
+    if (blk_expert != nullptr && blk_expert[t >> 7] < 0) continue;
     float g[8], u[8], d[8], dg[8], du[8];
     load8(gu + t * 2 * I + v * 8, g);
     load8(gu + t * 2 * I + I + v * 8, u);
@@ -406,20 +410,21 @@ static int rope_launch(void* q, void* k, long long q_stride, long long k_stride,
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
-extern "C" int vb_swiglu_fwd(const void* gu, void* out, long long T, int I, cudaStream_t stream) {
+extern "C" int vb_swiglu_fwd(const void* gu, void* out, long long T, int I, const int* blk_expert, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (I & 7) return -3;
   cudaError_t e = vb_launch_pdl(swiglu_fwd_kernel, dim3(grid_for(T * (I / 8), 256, 148 * 16)), dim3(256), 0, stream, 1,
-                                (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, I);
+                                (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, I, blk_expert);
   vb_count_launch();
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
-extern "C" int vb_swiglu_bwd(const void* gu, const void* dout, void* dgu, long long T, int I, cudaStream_t stream) {
+extern "C" int vb_swiglu_bwd(const void* gu, const void* dout, void* dgu, long long T, int I, const int* blk_expert,
+                             cudaStream_t stream) {
   if (T <= 0) return 0;
   if (I & 7) return -3;
   swiglu_bwd_kernel<<<grid_for(T * (I / 8), 256, 148 * 16), 256, 0, stream>>>(
-      (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dgu, T, I);
+      (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dgu, T, I, blk_expert);
   vb_count_launch();
   return (int)cudaGetLastError();
 }

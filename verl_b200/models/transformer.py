@@ -193,15 +193,9 @@ class MoEMLP(nn.Module):
 
     def _forward(self, x, x_router):
         T, H = x.shape
-        logits = self.gate(x_router).float()
-        probs = torch.softmax(logits, dim=-1)
-        if self.replay_routing is not None:
-            top_i = self.replay_routing
-            top_w = probs.gather(-1, top_i)
-        else:
-            top_w, top_i = torch.topk(probs, self.k, dim=-1)
-        if self.norm_topk:
-            top_w = top_w / top_w.sum(-1, keepdim=True)
+        from ..ops.moe import moe_gate
+
+        top_w, top_i = moe_gate(self.gate(x_router), self.k, self.norm_topk, self.replay_routing)
         if self.tp_group is not None:
             from ..parallel.tensor_parallel import copy_to_tp_region
 

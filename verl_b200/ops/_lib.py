@@ -37,8 +37,8 @@ _SIGS = {
     "vb_rmsnorm_bwd": ([P, P, P, P, P, P, P, P, I, L, I, P], I),
     "vb_rope": ([P, P, L, L, P, P, P, I, I, I, I, I, P], I),
     "vb_mrope": ([P, P, L, L, P, P, P, I, I, I, I, I, I, I, P], I),
-    "vb_swiglu_fwd": ([P, P, L, I, P], I),
-    "vb_swiglu_bwd": ([P, P, P, L, I, P], I),
+    "vb_swiglu_fwd": ([P, P, L, I, P, P], I),
+    "vb_swiglu_bwd": ([P, P, P, L, I, P, P], I),
     "vb_embedding_fwd": ([P, P, P, L, I, P], I),
     "vb_embedding_bwd": ([P, P, P, L, I, P], I),
     "vb_adamw": ([P, P, I, P, P, P, L, F, F, F, F, F, I, P, P, P], I),
@@ -62,6 +62,12 @@ _SIGS = {
     "vb_moe_route": ([P, L, I, I, I, I, I, P, P, P, P, P, I, P, P], I),
     "vb_moe_gather": ([P, L, P, P, I, I, I, P, P, I, P], I),
     "vb_moe_sum": ([P, P, P, I, P, L, P, L, P, L, P, P, P, F, P, I, I, F, I, P], I),
+    "vb_moe_gate": ([P, L, I, I, I, I, I, I, P, P, P], I),
+    "vb_moe_gate_bwd": ([P, L, I, I, I, I, I, P, P, P, P, P], I),
+    "vb_moe_place": ([P, L, I, I, P, P, P, I, P, P], I),
+    "vb_moe_rows": ([P, P, P, L, I, I, P, P], I),
+    "vb_moe_rows_bwd": ([P, P, P, P, P, L, I, I, P, P, P], I),
+    "vb_moe_weighted_sum": ([P, P, P, I, I, P, I, P], I),
     "vb_grouped_gemm_simt": ([P, P, P, I, I, I, P, I, P], I),
     "vb_rglru_tc_supported": ([I, I], I),
     "vb_rglru_conv": ([P, L, P, P, P, P, P, P, P, I, I, I, I, I, P], I),

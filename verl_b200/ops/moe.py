@@ -106,6 +106,11 @@ def moe_mlp(x: torch.Tensor, top_i: torch.Tensor, top_w: torch.Tensor, gate_up: 
     T, H = x.shape
     k = top_i.shape[1]
     E = gate_up.shape[0]
+    if _fused_mlp_ok(x, top_i, top_w, gate_up, down, swiglu):
+        first = expert_offset if num_experts is not None and num_experts != E else 0
+        if torch.is_grad_enabled() and any(t.requires_grad for t in (x, top_w, gate_up, down)):
+            return _RoutedMlpFn.apply(x, top_i, top_w, gate_up, down, first)
+        return _routed_mlp(x.contiguous(), top_i.contiguous(), top_w.contiguous(), gate_up, down, first)[0]
     if num_experts is not None and num_experts != E:
         local = top_i - expert_offset
         local = torch.where((local >= 0) & (local < E), local, torch.full_like(local, E))
@@ -121,6 +126,136 @@ def moe_mlp(x: torch.Tensor, top_i: torch.Tensor, top_w: torch.Tensor, gate_up: 
     out = grouped_linear(h, down, blk_expert, expert_off)
     picked = out.index_select(0, dest).view(T, k, H)
     return (picked * top_w.to(x.dtype).unsqueeze(-1)).sum(1)
+
+
+# -------------------------------------------------- gate and routed experts of the homogeneous models, forward and backward
+class _GateFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, logits, k, renorm, given):
+        idx, w = _gate(logits, k, renorm, given)
+        ctx.save_for_backward(logits, idx, w)
+        ctx.renorm = renorm
+        ctx.mark_non_differentiable(idx)
+        return w, idx
+
+    @staticmethod
+    def backward(ctx, g, _):
+        logits, idx, w = ctx.saved_tensors
+        (T, E), k = logits.shape, idx.shape[1]
+        dz = torch.empty((T, E), dtype=logits.dtype, device=logits.device)
+        g = g.contiguous()
+        rc = _lib.fn("vb_moe_gate_bwd")(logits.data_ptr(), logits.stride(0), T, E, k, int(ctx.renorm),
+                                        int(logits.dtype == torch.float32), idx.data_ptr(), w.data_ptr(), g.data_ptr(),
+                                        dz.data_ptr(), _lib.stream())
+        _lib.check(rc, "vb_moe_gate_bwd")
+        return dz, None, None, None
+
+
+def _gate(logits, k, renorm, given):
+    T, E = logits.shape
+    idx = given if given is not None else torch.empty((T, k), dtype=torch.long, device=logits.device)
+    w = torch.empty((T, k), dtype=torch.float32, device=logits.device)
+    rc = _lib.fn("vb_moe_gate")(logits.data_ptr(), logits.stride(0), T, E, k, int(renorm), int(given is not None),
+                                int(logits.dtype == torch.float32), idx.data_ptr(), w.data_ptr(), _lib.stream())
+    _lib.check(rc, "vb_moe_gate")
+    return idx, w
+
+
+def moe_gate(logits: torch.Tensor, k: int, renorm: bool, given: torch.Tensor | None = None):
+    """Softmax gate: (weights fp32 [T, k], experts int64 [T, k]) of the ``k`` most probable experts of every row of ``logits``
+    [T, E], or of the ``given`` ones (router replay). ``renorm``: the weights are divided by their sum."""
+    if (logits.is_cuda and logits.dtype in (torch.bfloat16, torch.float32) and logits.shape[1] <= 512 and k <= 32
+            and logits.stride(1) == 1 and (given is None or (given.dtype == torch.long and given.shape[1] == k))):
+        if given is not None:
+            given = given.contiguous()
+        if torch.is_grad_enabled() and logits.requires_grad:
+            return _GateFn.apply(logits, k, renorm, given)
+        idx, w = _gate(logits, k, renorm, given)
+        return w, idx
+    probs = torch.softmax(logits.float(), dim=-1)
+    if given is not None:
+        top_i, top_w = given, probs.gather(-1, given)
+    else:
+        top_w, top_i = torch.topk(probs, k, dim=-1)
+    return (top_w / top_w.sum(-1, keepdim=True) if renorm else top_w), top_i
+
+
+def _fused_mlp_ok(x, top_i, top_w, gate_up, down, swiglu) -> bool:
+    from . import nn
+
+    H, I2 = x.shape[1], gate_up.shape[1]
+    return (x.is_cuda and swiglu is nn.swiglu and x.shape[0] > 0 and x.dtype == gate_up.dtype == down.dtype == torch.bfloat16
+            and top_i.dtype == torch.long and top_w.dtype == torch.float32 and gate_up.shape[0] <= 2048 and H % 64 == 0
+            and I2 % 128 == 0 and gate_up.is_contiguous() and down.is_contiguous()
+            and gate_up.data_ptr() % 16 == 0 and down.data_ptr() % 16 == 0)
+
+
+def _routed_mlp(x, top_i, top_w, gate_up, down, first):
+    """x [T, H], top_i / top_w [T, k] contiguous, experts ``[first, first + E)`` -> (sum [T, H], what the backward needs).
+    Rows of blocks without an expert are never written; rows that pad an expert's share are zero in ``xs`` and so in ``h``."""
+    (T, H), k = x.shape, top_i.shape[1]
+    E, I2, _ = gate_up.shape
+    n, dev, stream = T * k, x.device, _lib.stream()
+    P = (n + min(E, n) * (BLK - 1)) // BLK * BLK
+    new = lambda *s, dt=torch.bfloat16: torch.empty(s, dtype=dt, device=dev)  # noqa: E731
+    dest, src, blk, off = (new(m, dt=torch.int32) for m in (n, P, P // BLK, E + 1))
+    rc = _lib.fn("vb_moe_place")(top_i.data_ptr(), n, first, E, dest.data_ptr(), src.data_ptr(), blk.data_ptr(), P // BLK,
+                                 off.data_ptr(), stream)
+    _lib.check(rc, "vb_moe_place")
+    xs = new(P, H)
+    _lib.check(_lib.fn("vb_moe_rows")(x.data_ptr(), src.data_ptr(), blk.data_ptr(), P, k, H, xs.data_ptr(), stream), "vb_moe_rows")
+    gu, h, out, y = new(P, I2), new(P, I2 // 2), new(P, H), new(T, H)
+    _grouped(xs, gate_up, gu, P, I2, H, False, False, False, 1, E, blk, None)
+    _lib.check(_lib.fn("vb_swiglu_fwd")(gu.data_ptr(), h.data_ptr(), P, I2 // 2, blk.data_ptr(), stream), "vb_swiglu_fwd")
+    _grouped(h, down, out, P, H, I2 // 2, False, False, False, 1, E, blk, None)
+    rc = _lib.fn("vb_moe_weighted_sum")(out.data_ptr(), dest.data_ptr(), top_w.data_ptr(), T, k, y.data_ptr(), H, stream)
+    _lib.check(rc, "vb_moe_weighted_sum")
+    return y, (xs, gu, h, out, dest, src, blk, off)
+
+
+class _RoutedMlpFn(torch.autograd.Function):
+    """:func:`_routed_mlp` with gradients. If the stacked weights have ``main_grad`` (fp32), their gradients are accumulated there."""
+
+    @staticmethod
+    def forward(ctx, x, top_i, top_w, gate_up, down, first):
+        x, top_i, top_w = x.contiguous(), top_i.contiguous(), top_w.contiguous()
+        y, kept = _routed_mlp(x, top_i, top_w, gate_up, down, first)
+        ctx.save_for_backward(top_w, gate_up, down, *kept)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        top_w, gate_up, down, xs, gu, h, out, dest, src, blk, off = ctx.saved_tensors
+        (T, k), (P, H), (E, I2, _) = top_w.shape, xs.shape, gate_up.shape
+        need_x, _, need_w, need_gu, need_down, _ = ctx.needs_input_grad
+        stream, dy = _lib.stream(), dy.contiguous()
+        new = lambda *s: torch.empty(s, dtype=torch.bfloat16, device=dy.device)  # noqa: E731
+
+        def weight_grad(weight, d, a):  # d^T a per expert
+            main = getattr(weight, "main_grad", None)
+            acc = main if main is not None else torch.zeros(weight.shape, dtype=torch.float32, device=dy.device)
+            _grouped(d, a, acc, d.shape[1], a.shape[1], P, True, True, True, 2, E, None, off)
+            return None if main is not None else acc.to(weight.dtype)
+
+        dw = torch.zeros((T, k), dtype=torch.float32, device=dy.device) if need_w else None
+        dout = new(P, H)
+        rc = _lib.fn("vb_moe_rows_bwd")(dy.data_ptr(), src.data_ptr(), blk.data_ptr(), top_w.data_ptr(), out.data_ptr(), P, k, H,
+                                        dout.data_ptr(), _lib.ptr(dw), stream)
+        _lib.check(rc, "vb_moe_rows_bwd")
+        d_down = weight_grad(down, dout, h) if need_down else None
+        dx = d_gate_up = None
+        if need_x or need_gu:
+            dh, dgu = new(P, I2 // 2), new(P, I2)
+            _grouped(dout, down, dh, P, I2 // 2, H, False, True, False, 1, E, blk, None)
+            rc = _lib.fn("vb_swiglu_bwd")(gu.data_ptr(), dh.data_ptr(), dgu.data_ptr(), P, I2 // 2, blk.data_ptr(), stream)
+            _lib.check(rc, "vb_swiglu_bwd")
+            d_gate_up = weight_grad(gate_up, dgu, xs) if need_gu else None
+            if need_x:
+                dxs, dx = new(P, H), new(T, H)
+                _grouped(dgu, gate_up, dxs, P, H, I2, False, True, False, 1, E, blk, None)
+                rc = _lib.fn("vb_moe_weighted_sum")(dxs.data_ptr(), dest.data_ptr(), None, T, k, dx.data_ptr(), H, stream)
+                _lib.check(rc, "vb_moe_weighted_sum")
+        return dx, None, dw, d_gate_up, d_down, None
 
 
 # ----------------------------------------------------------------- inference: routing, experts and their sum as fused kernels

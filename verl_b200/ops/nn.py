@@ -214,7 +214,7 @@ class _SwiGLUFn(torch.autograd.Function):
     def forward(ctx, gu):
         T, I2 = gu.shape
         out = torch.empty(T, I2 // 2, dtype=gu.dtype, device=gu.device)
-        rc = _lib.fn("vb_swiglu_fwd")(gu.data_ptr(), out.data_ptr(), T, I2 // 2, _lib.stream())
+        rc = _lib.fn("vb_swiglu_fwd")(gu.data_ptr(), out.data_ptr(), T, I2 // 2, None, _lib.stream())
         _lib.check(rc, "vb_swiglu_fwd")
         ctx.save_for_backward(gu)
         return out
@@ -225,7 +225,7 @@ class _SwiGLUFn(torch.autograd.Function):
         T, I2 = gu.shape
         dgu = torch.empty_like(gu)
         rc = _lib.fn("vb_swiglu_bwd")(gu.data_ptr(), dout.contiguous().data_ptr(), dgu.data_ptr(), T, I2 // 2,
-                                      _lib.stream())
+                                      None, _lib.stream())
         _lib.check(rc, "vb_swiglu_bwd")
         return dgu
 
