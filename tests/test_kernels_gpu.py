@@ -45,6 +45,26 @@ def test_gemm_layouts(mode, shape):
     _bf16_close(out, ref)
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 24, 25, 32, 33])
+@pytest.mark.parametrize("N,K", [(1, 8), (15, 72), (33, 520), (1153, 896), (4745, 2056), (130, 4872), (264, 8200), (37889, 64)])
+def test_gemm_few_rows(M, N, K):
+    """Few rows of A: every group of rows and of columns with its remainders, strided operands and results, both result types."""
+    from verl_b200.ops import gemm
+
+    torch.manual_seed(M * 7 + N)
+    A = torch.randn(M, K + 16, device="cuda").bfloat16()[:, 8 : K + 8]
+    B = torch.randn(N, K + 8, device="cuda").bfloat16()[:, :K]
+    bias = torch.randn(N, device="cuda").bfloat16()
+    ref = A.double() @ B.double().t()
+    # an fp32 sum of K products: at most K roundings of 2^-24 of the sum of their magnitudes
+    bound = (A.double().abs() @ B.double().abs().t()) * K * 2.0 ** -24
+    out = torch.full((M, N + 5), 7.0, device="cuda")
+    gemm(A, B, out=out[:, :N])
+    assert ((out[:, :N] - ref).abs() <= bound).all() and (out[:, N:] == 7.0).all()
+    got, want = gemm(A, B, bias=bias).double(), ref + bias.double()
+    assert ((got - want).abs() <= bound + 2.0 ** -8 * want.abs() + 2.0 ** -23).all()
+
+
 def test_gemm_fp32_accumulate_and_bias():
     from verl_b200.ops import gemm
 

@@ -1,0 +1,139 @@
+// C [M, N] = A [M, K] . B [N, K]^T (+ bias) for up to 32 rows of A: the projections of a decode step with few sequences.
+//
+// Bound by reading B once. The tcgen05 kernel has 128 rows per tile whatever M is, and its chain (barriers, tensor memory, TMA,
+// reduction of the K slices over a cluster) takes 7 us before a byte of B counts; here a block owns 16 * RT rows of B, its warps take
+// turns along K, and their sums meet in shared memory. Products run on mma.m16n8k16 with the rows of B as its 16 and the rows of A as
+// its 8: a lane's 16-byte loads are fragments as they come, since the order of k inside a product is free as long as both operands
+// share it. fp32 sums, as in the tcgen05 kernel. While the kernel before it runs, a block asks for its first rows of B in L2 (a hint,
+// so that it may come before the wait).
+#include "common.cuh"
+#include "host_utils.h"
+
+namespace vb {
+
+__device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {
+  uint4 v;
+  asm("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+constexpr int SK_WARPS = 8;
+
+// NT: groups of 8 rows of A; RT: groups of 16 rows of B per warp; UB: 64-wide steps of k whose loads are in flight together.
+template <int NT, int RT, int UB>
+__global__ void __launch_bounds__(SK_WARPS * 32, 2)
+gemm_skinny_kernel(const __nv_bfloat16* A, const __nv_bfloat16* B, void* __restrict__ C, const __nv_bfloat16* bias, int M, int N, int K,
+                   long long lda, long long ldb, long long ldc, int out_fp32) {
+  constexpr int ROWS = 16 * RT, COLS = 8 * NT;
+  __shared__ float red[SK_WARPS][ROWS][COLS + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n0 = blockIdx.x * ROWS;
+  pdl_trigger();
+  {
+    const int lines = (K + 63) >> 6;  // of 128 bytes per row
+    for (int i = threadIdx.x; i < ROWS * lines && i < 4 * SK_WARPS * 32; i += SK_WARPS * 32) {
+      const __nv_bfloat16* p = B + (long long)min(n0 + i % ROWS, N - 1) * ldb + (i / ROWS) * 64;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+    }
+  }
+  pdl_wait();
+  // rows past the ends repeat the last one: their sums are not stored
+  const __nv_bfloat16* b[RT * 2];
+  const __nv_bfloat16* a[NT];
+#pragma unroll
+  for (int r = 0; r < RT * 2; ++r) b[r] = B + (long long)min(n0 + r * 8 + g, N - 1) * ldb + t * 8;
+#pragma unroll
+  for (int j = 0; j < NT; ++j) a[j] = A + (long long)min(j * 8 + g, M - 1) * lda + t * 8;
+  float acc[RT][NT][4] = {};
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (int k0 = warp * 64; k0 < K; k0 += SK_WARPS * 64 * UB) {
+    uint4 w[UB][2][RT * 2], x[UB][2][NT];
+#pragma unroll
+    for (int u = 0; u < UB; ++u)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int k = k0 + u * (SK_WARPS * 64) + h * 32;
+        const bool in = k + t * 8 < K;  // K is a multiple of 8
+#pragma unroll
+        for (int r = 0; r < RT * 2; ++r) w[u][h][r] = in ? ld_stream(b[r] + k) : zero;
+#pragma unroll
+        for (int j = 0; j < NT; ++j) x[u][h][j] = in ? __ldg(reinterpret_cast<const uint4*>(a[j] + k)) : zero;
+      }
+#pragma unroll
+    for (int u = 0; u < UB; ++u)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+#pragma unroll
+          for (int j = 0; j < NT; ++j) {
+            const uint4 lo = w[u][h][2 * r], hi = w[u][h][2 * r + 1], v = x[u][h][j];
+            mma_16816(acc[r][j], lo.x, hi.x, lo.y, hi.y, v.x, v.y);
+            mma_16816(acc[r][j], lo.z, hi.z, lo.w, hi.w, v.z, v.w);
+          }
+  }
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) red[warp][r * 16 + (i >> 1) * 8 + g][j * 8 + 2 * t + (i & 1)] = acc[r][j][i];
+  __syncthreads();
+  for (int i = threadIdx.x; i < ROWS * COLS; i += SK_WARPS * 32) {
+    const int n = n0 + i % ROWS, m = i / ROWS;
+    if (n >= N || m >= M) continue;
+    float s = 0.f;
+#pragma unroll
+    for (int v = 0; v < SK_WARPS; ++v) s += red[v][i % ROWS][m];
+    if (bias) s += __bfloat162float(bias[n]);
+    if (out_fp32) reinterpret_cast<float*>(C)[m * ldc + n] = s;
+    else reinterpret_cast<__nv_bfloat16*>(C)[m * ldc + n] = __float2bfloat16(s);
+  }
+}
+
+}  // namespace vb
+
+using namespace vb;
+
+// Measured against the tcgen05 kernel, chains of launches on alternating matrices (us, M = 1 / 16 / 24 / 32; its own in brackets):
+//   896 -> 1152    2.3 / 2.6 / 3.1 / 3.3 (6.8)           3584 -> 4608   6.5 / 7.9 / 8.9 / 10.3 (17.4, at 24 and 32: 15.3)
+//   896 -> 9728    5.6 / 6.2 / 8.0 / 9.1 (14.6, 12.7)    2048 -> 5120   5.2 / 7.2 / 8.1 / 9.3 (13.5)
+//   3584 -> 37888  45 / 59 / 67 / 81 (66 / 52 / 46 / 46)  18944 -> 3584  23 / 27 / 32 / 40 (30 to 38)
+// Beyond 8 rows the loads of A (from L2, by every block) grow to those of B: where tiles of the tcgen05 kernel fill all SMs it is as
+// fast at 16 rows and faster beyond, and with long rows (K) its staged operands win from 24 and 32 rows on.
+bool vb_gemm_skinny_ok(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B);
+  if ((K & 7) || (lda & 7) || (ldb & 7) || (at & 15)) return false;
+  if (M <= 8) return true;
+  if (N >= 256 * vb_num_sms()) return false;
+  return M <= 16 || (M <= 24 && K <= 8192) || (M <= 32 && K <= 4096);
+}
+
+extern "C" int vb_gemm_skinny(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, long long lda,
+                              long long ldb, long long ldc, int out_fp32, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (!vb_gemm_skinny_ok(A, B, M, N, K, lda, ldb)) return -3;
+  cudaError_t e;
+#define VB_SKINNY(NT, RT, UB)                                                                                              \
+  e = vb_launch_pdl(gemm_skinny_kernel<NT, RT, UB>, dim3((N + 16 * RT - 1) / (16 * RT)), dim3(SK_WARPS * 32), 0, stream, 1, \
+                    (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, C, (const __nv_bfloat16*)bias, M, N, K, lda, ldb, ldc, \
+                    out_fp32)
+  // 32 rows of B per block halve the loads of A; taken when the blocks still fill the SMs and their rows are long enough
+  // (2048 -> 5120 at 32 rows: 9.3 us against 12.3; 3584 -> 4608, 144 blocks: 13.1 against 10.3)
+  const bool two = N >= 32 * vb_num_sms() && K >= 2048;
+  if (M <= 8) VB_SKINNY(1, 1, 4);
+  else if (M <= 16 && two) VB_SKINNY(2, 2, 2);
+  else if (M <= 16) VB_SKINNY(2, 1, 2);
+  else if (M <= 24 && two) VB_SKINNY(3, 2, 1);
+  else if (M <= 24) VB_SKINNY(3, 1, 1);
+  else if (two) VB_SKINNY(4, 2, 1);
+  else VB_SKINNY(4, 1, 1);
+#undef VB_SKINNY
+  vb_count_launch();
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}

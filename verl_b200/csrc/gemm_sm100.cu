@@ -1181,6 +1181,11 @@ static int max_active_clusters(int bn, int cluster) {
 
 using namespace vb;
 
+// gemm_skinny.cu
+bool vb_gemm_skinny_ok(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb);
+extern "C" int vb_gemm_skinny(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, long long lda,
+                              long long ldb, long long ldc, int out_fp32, cudaStream_t stream);
+
 // C[M,N] = A . B^T, bf16 inputs, fp32 accumulation.
 //   a_mn = 0: A is [M,K] row-major (lda elements per row); a_mn = 1: A is stored [K,M] row-major.
 //   b_mn = 0: B is [N,K] row-major;                         b_mn = 1: B is stored [K,N] row-major.
@@ -1196,6 +1201,8 @@ static int gemm_bf16_run(const void* A, const void* B, void* C, const void* bias
                          int* status, cudaStream_t stream, void* const* rs_dst, int rs_world, int rs_rows) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7)) return -3;
+  if (!a_mn && !b_mn && !accumulate && rs_dst == nullptr && vb_gemm_skinny_ok(A, B, M, N, K, lda, ldb))
+    return vb_gemm_skinny(A, B, C, bias, M, N, K, lda, ldb, ldc, out_fp32, stream);
   GemmParams p{};
   p.M = M; p.N = N; p.K = K;
   p.C = C; p.ldc = ldc; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
