@@ -403,7 +403,8 @@ def test_sampler_never_takes_a_token_of_no_weight():
 
 @pytest.mark.parametrize("B,Hq,Hk,D,bs,maxlen", [(5, 28, 4, 128, 16, 700), (3, 4, 2, 64, 16, 300), (2, 32, 4, 128, 32, 3000),
                                                  (4, 40, 8, 128, 16, 150), (3, 32, 2, 128, 128, 1000),
-                                                 (2, 8, 8, 128, 8, 260),
+                                                 (2, 8, 8, 128, 8, 260), (1, 14, 2, 64, 16, 110), (7, 8, 8, 64, 8, 129),
+                                                 (3, 32, 2, 64, 32, 1025), (40, 8, 1, 64, 256, 2100), (3, 9, 1, 128, 16, 513),
                                                  # more (sequence, head, split) items than resident CTAs: the
                                                  # persistent kernel (CTAs walk several items, some of them empty)
                                                  (100, 28, 4, 128, 16, 700), (80, 32, 8, 128, 16, 300)])
@@ -430,7 +431,7 @@ def test_paged_decode_attention(B, Hq, Hk, D, bs, maxlen):
     ref = ops.paged_decode_attention(q.cpu().float(), kc.cpu().float(), vc.cpu().float(), table.cpu(), lens)
     from verl_b200.ops import _lib
 
-    impls = ["simt"] if Hq // Hk <= 8 else []
+    impls = ["auto"] + (["simt"] if Hq // Hk <= 8 else [])
     if _lib.fn("vb_paged_decode_tc_supported")(Hq, Hk, D, bs):
         impls.append("tc")
     assert impls

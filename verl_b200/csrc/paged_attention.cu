@@ -191,8 +191,10 @@ paged_decode_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,  //
 }
 
 template <int D>
-__global__ void decode_merge_kernel(const float* __restrict__ o_part, const float* __restrict__ ml_part, int Hq,
-                                    int num_splits, __nv_bfloat16* __restrict__ out, long long out_stride) {
+__global__ void decode_merge_kernel(const float* o_part, const float* ml_part, int Hq, int num_splits,
+                                    __nv_bfloat16* __restrict__ out, long long out_stride) {
+  pdl_trigger();
+  pdl_wait();
   const int b = blockIdx.x, hq = blockIdx.y, d = threadIdx.x;
   const long long base = ((long long)b * Hq + hq) * num_splits;
   float m = -INFINITY;
@@ -289,12 +291,13 @@ extern "C" int vb_decode_num_splits(int B, int Hk, int max_seq_len) {
   return s;
 }
 
-// Merge of the per-split partial results (head_dim 128), shared with the tensor-core decode kernel.
-int vb_decode_merge_128(const float* o_part, const float* ml_part, int B, int Hq, int num_splits, void* out,
-                        long long out_stride, cudaStream_t stream) {
-  decode_merge_kernel<128><<<dim3(B, Hq), 128, 0, stream>>>(o_part, ml_part, Hq, num_splits, (__nv_bfloat16*)out,
-                                                            out_stride);
-  return (int)cudaGetLastError();
+// Merge of the per-split partial results, D 64 or 128.
+int vb_decode_merge_parts(const float* o_part, const float* ml_part, int B, int Hq, int D, int num_splits, void* out, long long out_stride,
+                          cudaStream_t stream) {
+  const cudaError_t e =
+      vb_launch_pdl(D == 128 ? decode_merge_kernel<128> : decode_merge_kernel<64>, dim3(B, Hq), dim3(D), 0, stream, 1, o_part, ml_part, Hq,
+                    num_splits, (__nv_bfloat16*)out, out_stride);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
 int vb_decode_merge(const float* o_part, const float* ml_part, int B, int Hq, int D, int num_splits, void* out,
@@ -319,22 +322,18 @@ extern "C" int vb_paged_decode(const void* q, long long q_stride, const void* kc
                                                        (const __nv_bfloat16*)vc, block_table, max_blocks, seq_lens,
                                                        Hq, Hk, block_size, scale, num_splits, (__nv_bfloat16*)out,
                                                        out_stride, o_part, ml_part);
-    if (num_splits > 1)
-      decode_merge_kernel<128><<<dim3(B, Hq), 128, 0, stream>>>(o_part, ml_part, Hq, num_splits, (__nv_bfloat16*)out,
-                                                                out_stride);
   } else if (D == 64) {
     paged_decode_kernel<64><<<grid, 128, 0, stream>>>((const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)kc,
                                                       (const __nv_bfloat16*)vc, block_table, max_blocks, seq_lens, Hq,
                                                       Hk, block_size, scale, num_splits, (__nv_bfloat16*)out,
                                                       out_stride, o_part, ml_part);
-    if (num_splits > 1)
-      decode_merge_kernel<64><<<dim3(B, Hq), 64, 0, stream>>>(o_part, ml_part, Hq, num_splits, (__nv_bfloat16*)out,
-                                                              out_stride);
   } else {
     return -3;
   }
   vb_count_launch(num_splits > 1 ? 2 : 1);
-  return (int)cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || num_splits == 1) return (int)e;
+  return vb_decode_merge_parts(o_part, ml_part, B, Hq, D, num_splits, out, out_stride, stream);
 }
 
 extern "C" int vb_kv_cache_write(const void* k, const void* v, long long k_stride, long long v_stride,

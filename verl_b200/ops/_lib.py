@@ -109,7 +109,8 @@ _SIGS = {
     "vb_flash_bwd_dkv": ([P, P, P, P, L, L, L, L, P, I, L, I, I, I, F, I, P, P, P, P, L, P, P], I),
     "vb_flash_fwd": ([P, P, P, L, L, L, P, P, I, L, L, I, I, I, F, I, P, L, P, P, P], I),
     "vb_paged_decode_tc_supported": ([I, I, I, I], I),
-    "vb_paged_decode_tc": ([P, L, P, P, I, P, I, P, I, I, I, I, F, I, P, L, P, P, P], I),
+    "vb_paged_decode_mma_supported": ([I, I, I, I], I),
+    "vb_paged_decode_mma": ([P, L, P, P, P, I, P, I, I, I, I, I, F, I, P, L, P, P], I),
     "vb_paged_decode": ([P, L, P, P, P, I, P, I, I, I, I, I, F, I, P, L, P, P], I),
     "vb_kv_cache_write": ([P, P, L, L, P, P, P, L, I, I, I, P], I),
 }

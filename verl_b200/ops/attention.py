@@ -166,8 +166,8 @@ def paged_decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
     """One query token per sequence. q [B,Hq,D]; caches [NB,Hk,BS,D]; block_table int32 [B,max_blocks];
     seq_lens int32 [B] (including the current token, already written to the cache).
 
-    ``impl``: "tc" = tcgen05 kernel (head_dim 128, <= 16 query heads per KV head, block size a power of two in
-    8..128), "simt" = CUDA-core kernel, "auto" = "tc" wherever it applies."""
+    ``impl``: "tc" = tensor-core kernel (head_dim 128, <= 16 query heads per KV head, block size a power of two in
+    8..128), "simt" = CUDA-core kernel, "auto" = the tensor-core kernel wherever it applies."""
     B, Hq, D = q.shape
     Hk, BS = k_cache.shape[1], k_cache.shape[2]
     scale = scale if scale is not None else D ** -0.5
@@ -179,19 +179,14 @@ def paged_decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
         tc_ok = bool(_lib.fn("vb_paged_decode_tc_supported")(Hq, Hk, D, BS)) and k_cache.is_contiguous() and v_cache.is_contiguous()
         if impl == "tc" and not tc_ok:
             raise ValueError(f"tensor-core decode does not support Hq={Hq} Hk={Hk} D={D} block_size={BS}")
-        if tc_ok and impl != "simt":
-            rc = _lib.fn("vb_paged_decode_tc")(q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
-                                               k_cache.shape[0], block_table.data_ptr(), block_table.stride(0),
-                                               seq_lens.data_ptr(), B, Hq, Hk, BS, scale, num_splits, out.data_ptr(),
-                                               out.stride(0), _lib.ptr(work), _lib.status_word(q.device).data_ptr(),
-                                               _lib.stream())
-            _lib.check(rc, "vb_paged_decode_tc")
-            return out
-        rc = _lib.fn("vb_paged_decode")(q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
-                                        block_table.data_ptr(), block_table.stride(0), seq_lens.data_ptr(), B, Hq, Hk,
-                                        D, BS, scale, num_splits, out.data_ptr(), out.stride(0), _lib.ptr(work),
-                                        _lib.stream())
-        _lib.check(rc, "vb_paged_decode")
+        # auto: heads of 64 and larger blocks too, wherever the tensor-core kernel takes the caches
+        name = "vb_paged_decode_mma" if impl != "simt" and (tc_ok or (
+            k_cache.is_contiguous() and v_cache.is_contiguous() and (k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0
+            and bool(_lib.fn("vb_paged_decode_mma_supported")(Hq, Hk, D, BS)))) else "vb_paged_decode"
+        rc = _lib.fn(name)(q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), block_table.data_ptr(),
+                           block_table.stride(0), seq_lens.data_ptr(), B, Hq, Hk, D, BS, scale, num_splits, out.data_ptr(),
+                           out.stride(0), _lib.ptr(work), _lib.stream())
+        _lib.check(rc, name)
         return out
     G = Hq // Hk
     for b in range(B):
