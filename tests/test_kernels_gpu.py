@@ -670,7 +670,12 @@ def test_bounded_device_wait_reports_status_and_context_survives():
     _bf16_close(gemm(a, a), a.float() @ a.float().t())
 
 
-@pytest.mark.parametrize("M,N,K,pow2", [(128, 512, 1024, False), (300, 384 + 64, 640, True), (1000, 256, 3584, False)])
+@pytest.mark.parametrize("M,N,K,pow2", [(128, 512, 1024, False), (300, 384 + 64, 640, True), (1000, 256, 3584, False),
+                                        # decode: every width of the tile, one CTA and up to eight per tile, uneven shares of K
+                                        (1, 128, 128, False), (16, 200, 1040, False), (17, 1152, 896, False), (32, 64, 4864, False),
+                                        (33, 3584, 3584, False), (48, 4608, 3584, False), (49, 130, 144, False),
+                                        (64, 896, 18944, False), (65, 37888, 512, False), (65, 520, 3584, False),
+                                        (127, 3584, 3600, False)])
 def test_fp8_blockscale_quant_and_gemm(M, N, K, pow2):
     from verl_b200.ops import _lib, fp8
 

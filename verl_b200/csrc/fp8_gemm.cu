@@ -13,6 +13,9 @@
 // epilogue warps read the partial, multiply by the two scales and accumulate in registers while the MMA of the
 // next k block runs into the other buffer ("promotion" of every 128-deep partial sum to fp32 outside the tensor
 // core, which is what block scaling with plain fp32 scales requires).
+//
+// Up to 128 rows of X (decode steps) take fp8_gemm_skinny_kernel: W's rows are the MMA's 128 rows and X's rows its columns, so that the
+// promotion costs a column per row of X instead of 128, and the CTAs of a cluster share a tile's K.
 #include "common.cuh"
 #include "host_utils.h"
 
@@ -67,6 +70,8 @@ __global__ void fp8_quant_weight_kernel(const __nv_bfloat16* __restrict__ w, lon
 // one warp per (row, 128-column block)
 __global__ void fp8_quant_act_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, long long M, int K,
                                      __nv_fp8_storage_t* __restrict__ q, long long ldq, float* __restrict__ scales, int pow2) {
+  pdl_trigger();
+  pdl_wait();
   const int nkb = (K + 127) / 128;
   const long long unit = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (unit >= M * nkb) return;
@@ -269,6 +274,300 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   }
 }
 
+// ------------------------------------------------------------------------------------------------ decode
+// C^T tile [128 rows of W, NT rows of X] per cluster of `splits` CTAs, each with its part of the k blocks. What bounds it is reading W
+// once; the kernel above read 68 MB on 28 SMs with a promotion of 128 columns per k block (48 rows of X; 18 944 -> 3584: 69 us, now
+// 25, floor 11). Partial products wait in F8S_BUFS tensor-memory buffers; the fp32 sums of a cluster meet in shared memory, in slice
+// order. The first rows of W are asked for in L2 while the kernel before still runs (a hint, it may come before the wait).
+constexpr int F8S_BUFS = 4;
+template <int NT>
+struct F8Skinny {
+  static_assert(NT <= 64 && NT % 16 == 0, "two CTAs per SM");
+  static constexpr int COLS = NT <= 32 ? 32 : 64;  // tensor-memory columns of a buffer
+  static constexpr int BUFS = F8S_BUFS;
+  static constexpr int STAGE = F8_TILE + NT * 128;
+  static constexpr int STAGES = NT <= 32 ? 5 : 4;
+  static constexpr int SCALE_OFF = STAGES * STAGE;                  // [4 warps][2][NT] fp32
+  static constexpr int BAR_OFF = SCALE_OFF + 4 * 2 * NT * 4;
+  static constexpr int SMEM = BAR_OFF + (2 * STAGES + 2 * BUFS) * 8 + 16 + 1024;
+  static_assert(NT * 128 * 4 <= STAGES * STAGE, "the partial tile takes the stages' place");
+};
+
+template <int NT>
+__global__ void __launch_bounds__(F8_THREADS, 2)
+fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const F8Params p,
+                       const uint8_t* w, long long ldw, int m_tiles, int splits, int kb_per) {
+  using L = F8Skinny<NT>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  float* scale_s = reinterpret_cast<float*>(smem + L::SCALE_OFF);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
+  uint64_t* empty = full + L::STAGES;
+  uint64_t* pfull = empty + L::STAGES;  // the product of a k block is in TMEM buffer i
+  uint64_t* pempty = pfull + L::BUFS;   // the epilogue warps have read buffer i
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pempty + L::BUFS);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int num_kb = (p.K + F8_BK - 1) / F8_BK;
+  const int rank = blockIdx.x % splits, nb = blockIdx.x / splits / m_tiles, m0 = blockIdx.x / splits % m_tiles * NT;
+  const int kb0 = rank * kb_per, kb1 = min(num_kb, kb0 + kb_per);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < L::STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int i = 0; i < L::BUFS; ++i) {
+      mbar_init(&pfull[i], 1);
+      mbar_init(&pempty[i], 4);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, L::BUFS * L::COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();  // TMEM is held
+  if (warp >= 2) {
+    const int n = nb * F8_BN + (int)threadIdx.x - 64;  // a row of W per thread
+    if (n < p.N)
+      for (int kb = kb0; kb < min(kb1, kb0 + L::STAGES); ++kb)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(w + (long long)n * ldw + kb * F8_BK));
+  }
+  pdl_wait();
+
+  bool ok = true;
+  if (warp == 0) {
+    if (lane == 0) {
+      tma_prefetch_desc(&tmW);
+      tma_prefetch_desc(&tmX);
+      int s = 0, issued = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (*abort_flag || !mbar_wait(&empty[s], phase ^ 1)) {
+          report_error(p.status, ERR_WAIT_EMPTY, kb);
+          *abort_flag = 1;
+          break;
+        }
+        mbar_arrive_expect_tx(&full[s], L::STAGE);
+        tma_load_2d(smem + s * L::STAGE, &tmW, &full[s], kb * F8_BK, nb * F8_BN);
+        tma_load_2d(smem + s * L::STAGE + F8_TILE, &tmX, &full[s], kb * F8_BK, m0);
+        ++issued;
+        if (++s == L::STAGES) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+      // no copy outlives the CTA (after an error; else they have all been waited for)
+      for (int i = max(0, issued - L::STAGES); i < issued; ++i) mbar_wait(&full[i % L::STAGES], (uint32_t)((i / L::STAGES) & 1));
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = umma_idesc(0, 0, 0, 0, 128, NT);
+      int s = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int it = kb - kb0, buf = it % L::BUFS;
+        if (*abort_flag || !mbar_wait(&pempty[buf], (uint32_t)((it / L::BUFS) & 1) ^ 1) || !mbar_wait(&full[s], phase)) {
+          report_error(p.status, ERR_WAIT_FULL, kb);
+          *abort_flag = 1;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t w_addr = smem_u32(smem + s * L::STAGE), x_addr = w_addr + F8_TILE;
+#pragma unroll
+        for (int k = 0; k < F8_BK / 32; ++k)
+          tc_mma_f8(tmem_base + buf * L::COLS, umma_smem_desc(w_addr + k * 32, 16, 1024), umma_smem_desc(x_addr + k * 32, 16, 1024),
+                    idesc, k != 0);
+        tc_commit(&empty[s]);
+        tc_commit(&pfull[buf]);
+        if (++s == L::STAGES) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
+    }
+    __syncwarp();
+  }
+  float acc[NT];
+  const int quad = warp & 3, row = quad * 32 + lane;  // row of the tile of W
+  if (warp >= 2) {
+    const uint32_t t_row = tmem_base + (((uint32_t)(quad * 32)) << 16);
+    float* sc = scale_s + quad * 2 * NT;
+#pragma unroll
+    for (int i = 0; i < NT; ++i) acc[i] = 0.f;
+    float next[(NT + 31) / 32];
+    auto fetch = [&](int kb) {  // the scales of k block kb: of X's rows, a row per lane, times that of the tile of W
+      if (kb >= kb1) return;
+      const float sw = p.sw[(long long)nb * num_kb + kb];
+#pragma unroll
+      for (int j = 0; j < (NT + 31) / 32; ++j) {
+        const int m = m0 + j * 32 + lane;
+        next[j] = j * 32 + lane < NT && m < p.M ? p.sx[(long long)m * num_kb + kb] * sw : 0.f;
+      }
+    };
+    fetch(kb0);
+    for (int kb = kb0; kb < kb1; ++kb) {
+      const int it = kb - kb0, buf = it % L::BUFS;
+      float* mine = sc + (it & 1) * NT;  // read by this warp in the turn before the last: every lane has passed a barrier since
+#pragma unroll
+      for (int j = 0; j < (NT + 31) / 32; ++j)
+        if (j * 32 + lane < NT) mine[j * 32 + lane] = next[j];
+      __syncwarp();
+      fetch(kb + 1);
+      if (*abort_flag || !mbar_wait(&pfull[buf], (uint32_t)((it / L::BUFS) & 1))) {
+        report_error(p.status, ERR_WAIT_TMEM_FULL, kb);
+        *abort_flag = 1;
+        ok = false;
+        break;
+      }
+      __syncwarp();
+      tc_fence_after();
+      uint32_t v[NT / 16][16];
+#pragma unroll
+      for (int c = 0; c < NT / 16; ++c) tmem_ld_32x16(t_row + buf * L::COLS + c * 16, v[c]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < NT; i += 4) {
+        const float4 f = *reinterpret_cast<const float4*>(mine + i);
+        acc[i] = fmaf(__uint_as_float(v[i / 16][i % 16]), f.x, acc[i]);
+        acc[i + 1] = fmaf(__uint_as_float(v[i / 16][i % 16 + 1]), f.y, acc[i + 1]);
+        acc[i + 2] = fmaf(__uint_as_float(v[i / 16][i % 16 + 2]), f.z, acc[i + 2]);
+        acc[i + 3] = fmaf(__uint_as_float(v[i / 16][i % 16 + 3]), f.w, acc[i + 3]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&pempty[buf]);
+    }
+  }
+  const int rows = min(NT, p.M - m0);
+  if (splits == 1) {
+    const int n = nb * F8_BN + row;
+    if (warp >= 2 && ok && n < p.N) {
+      const float b = p.bias ? __bfloat162float(p.bias[n]) : 0.f;
+#pragma unroll
+      for (int m = 0; m < NT; ++m)
+        if (m < rows) p.C[(long long)(m0 + m) * p.ldc + n] = __float2bfloat16(acc[m] + b);
+    }
+  } else {
+    // all products of this CTA have been read, so its stages are idle: [NT][128] fp32
+    float* part = reinterpret_cast<float*>(smem);
+    __syncthreads();
+    if (warp >= 2) {
+#pragma unroll
+      for (int m = 0; m < NT; ++m) part[m * 128 + row] = acc[m];
+    }
+    cluster_sync_all();
+    // a warp per row of X, four columns per lane, the loads of all slices in flight together
+    const int n = nb * F8_BN + lane * 4;
+    float b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) b[i] = p.bias && n + i < p.N ? __bfloat162float(p.bias[n + i]) : 0.f;
+    const bool whole = n + 4 <= p.N && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 7) == 0;
+    for (int m = rank + splits * warp; m < rows; m += splits * (F8_THREADS / 32)) {
+      const uint32_t at = smem_u32(part + m * 128 + lane * 4);
+      float4 v[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (r < splits)
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(v[r].x), "=f"(v[r].y), "=f"(v[r].z), "=f"(v[r].w)
+                       : "r"(map_to_cta(at, r)));
+      float sum[4] = {};
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (r < splits) {
+          sum[0] += v[r].x;
+          sum[1] += v[r].y;
+          sum[2] += v[r].z;
+          sum[3] += v[r].w;
+        }
+      __nv_bfloat16* c = p.C + (long long)(m0 + m) * p.ldc + n;
+      if (whole) {
+        *reinterpret_cast<uint2*>(c) = make_uint2(pack_bf16x2(sum[0] + b[0], sum[1] + b[1]), pack_bf16x2(sum[2] + b[2], sum[3] + b[3]));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (n + i < p.N) c[i] = __float2bfloat16(sum[i] + b[i]);
+      }
+    }
+    cluster_sync_all();  // the others have read this CTA's part
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, L::BUFS * L::COLS);
+  }
+}
+
+// How many clusters of `cluster` CTAs of the kernel the device holds at once (asked once per size and device).
+template <int NT>
+static int fp8_skinny_clusters(int cluster) {
+  static int cache[64][9];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (cache[dev][cluster] == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cluster * 64);
+    cfg.blockDim = dim3(F8_THREADS);
+    cfg.dynamicSmemBytes = F8Skinny<NT>::SMEM;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = cluster;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, fp8_gemm_skinny_kernel<NT>, &cfg) != cudaSuccess || n <= 0) {
+      (void)cudaGetLastError();
+      n = -1;
+    }
+    cache[dev][cluster] = n;
+  }
+  return cache[dev][cluster];
+}
+
+template <int NT>
+static int launch_fp8_skinny(const void* xq, const void* wq, long long ldx, long long ldw, const F8Params& p, cudaStream_t stream) {
+  using L = F8Skinny<NT>;
+  CUtensorMap tmW, tmX;
+  int rc = vb_make_tmap_2d(&tmW, wq, 1, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)ldw, F8_BK, 128);
+  if (rc) return rc;
+  rc = vb_make_tmap_2d(&tmX, xq, 1, (uint64_t)p.K, (uint64_t)p.M, (uint64_t)ldx, F8_BK, NT);
+  if (rc) return rc;
+  auto kern = fp8_gemm_skinny_kernel<NT>;
+  static bool attr_set[64] = {};
+  int dev = 0;
+  VB_CUDA_CHECK(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+    VB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM));
+    if (dev >= 0 && dev < 64) attr_set[dev] = true;
+  }
+  // the most CTAs of one wave (two per SM), six k blocks or more per CTA: below, the cluster's exchange costs more than it gives
+  const int m_tiles = (p.M + NT - 1) / NT, tiles = (p.N + 127) / 128 * m_tiles, nkb = (p.K + F8_BK - 1) / F8_BK;
+  int splits = 1, per = nkb;
+  for (int s = 2; s <= 8 && s * 6 <= nkb && tiles * s <= 2 * vb_num_sms(); ++s) {
+    const int each = (nkb + s - 1) / s;
+    if ((nkb + each - 1) / each != s || tiles > fp8_skinny_clusters<NT>(s)) continue;
+    splits = s;
+    per = each;
+  }
+  cudaError_t e = vb_launch_ex(kern, dim3(tiles * splits), dim3(F8_THREADS), L::SMEM, stream, (unsigned)splits, true, tmW, tmX, p,
+                               (const uint8_t*)wq, ldw, m_tiles, splits, per);
+  vb_count_launch();
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
 }  // namespace vb
 
 using namespace vb;
@@ -289,10 +588,11 @@ extern "C" int vb_fp8_quant_act(const void* x, long long ldx, long long M, int K
                                 int pow2, cudaStream_t stream) {
   if (M <= 0 || K <= 0) return 0;
   const long long units = M * ((K + 127) / 128);
-  fp8_quant_act_kernel<<<(unsigned)((units + 7) / 8), 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(x), ldx, M, K,
-                                                                       reinterpret_cast<__nv_fp8_storage_t*>(q), ldq, scales, pow2);
+  cudaError_t e = vb_launch_pdl(fp8_quant_act_kernel, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, stream, 1,
+                                reinterpret_cast<const __nv_bfloat16*>(x), ldx, M, K, reinterpret_cast<__nv_fp8_storage_t*>(q), ldq,
+                                scales, pow2);
   vb_count_launch();
-  return (int)cudaGetLastError();
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
 // C [M, N] bf16 = dequantised Xq . Wq^T (+ bias). Xq [M, K], Wq [N, K] e4m3 with row strides (bytes = elements)
@@ -302,6 +602,21 @@ extern "C" int vb_fp8_gemm_blockscale(const void* xq, const void* wq, const floa
                                       int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((ldx & 15) || (ldw & 15)) return -3;
+  F8Params p{};
+  p.M = M; p.N = N; p.K = K;
+  p.C = reinterpret_cast<__nv_bfloat16*>(C); p.ldc = ldc;
+  p.sx = sx; p.sw = sw; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias); p.status = status;
+  // us, the kernel below -> the decode kernel (M = 1 / 48 / 64 / 96 / 128):
+  //   3584 -> 4608   16 -> 7.7 / 10 / 12 / 12 / 14    18944 -> 3584  68 -> 19 / 25 / 31 / 45 / 57    4096 -> 6144  18 -> 10 / 13 / 16 / 22 / 27
+  //   3584 -> 37888  36 -> 23 / 26 / 28 / 41 / 48     4096 -> 28672  40 -> 21 / 27 / 32 / 49 / 61    4864 -> 896   20 -> 6.1 / 7.6 / 8.3 / 8.2 / 9.5
+  // More than 64 rows of X are two tiles, which read W twice (from L2): worth it while all tiles together leave half of the SMs
+  // without one, so that the kernel below would, too.
+  if (M <= 16) return launch_fp8_skinny<16>(xq, wq, ldx, ldw, p, stream);
+  if (M <= 32) return launch_fp8_skinny<32>(xq, wq, ldx, ldw, p, stream);
+  if (M <= 48) return launch_fp8_skinny<48>(xq, wq, ldx, ldw, p, stream);
+  if (M <= 64) return launch_fp8_skinny<64>(xq, wq, ldx, ldw, p, stream);
+  if (M <= 128 && (N + 127) / 128 * 4 <= vb_num_sms())
+    return M <= 96 ? launch_fp8_skinny<48>(xq, wq, ldx, ldw, p, stream) : launch_fp8_skinny<64>(xq, wq, ldx, ldw, p, stream);
   CUtensorMap tmA, tmB;
   int rc = vb_make_tmap_2d(&tmA, xq, 1, (uint64_t)K, (uint64_t)M, (uint64_t)ldx, F8_BK, F8_BM);
   if (rc) return rc;
@@ -312,10 +627,6 @@ extern "C" int vb_fp8_gemm_blockscale(const void* xq, const void* wq, const floa
     VB_CUDA_CHECK(cudaFuncSetAttribute(fp8_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F8_SMEM));
     attr_set = true;
   }
-  F8Params p{};
-  p.M = M; p.N = N; p.K = K;
-  p.C = reinterpret_cast<__nv_bfloat16*>(C); p.ldc = ldc;
-  p.sx = sx; p.sw = sw; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias); p.status = status;
   const int tiles = ((M + F8_BM - 1) / F8_BM) * ((N + F8_BN - 1) / F8_BN);
   const int grid = tiles < vb_num_sms() ? tiles : vb_num_sms();
   fp8_gemm_kernel<<<grid, F8_THREADS, F8_SMEM, stream>>>(tmA, tmB, p);
