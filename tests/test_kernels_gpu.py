@@ -618,6 +618,29 @@ def test_routed_mlp_forms(T, E, k, H, I, first, total):
         assert err <= roundings * 2.0 ** -8 * float(want.abs().max()) + 1e-12, (got.shape, err, float(want.abs().max()))
 
 
+def test_routed_mlp_refuses_and_realigns():
+    """Routing of another number of tokens is refused before a kernel reads past it; rows and gradients off a 16-byte boundary work."""
+    from verl_b200 import ops
+    from verl_b200.ops.moe import moe_gate, moe_mlp
+
+    T, E, k, H, I = 20, 4, 2, 64, 64
+    gate_up, down = (torch.randn(*s, device="cuda").bfloat16() * 0.1 for s in ((E, 2 * I, H), (E, H, I)))
+    z = torch.randn(T, E, device="cuda")
+    w, idx = moe_gate(z, k, True)
+    x = torch.randn(T * H + 1, device="cuda").bfloat16()
+    off = x[1:].view(T, H)
+    y = moe_mlp(off, idx, w, gate_up, down, ops.swiglu)
+    _bf16_close(y, moe_mlp(off.clone(), idx, w, gate_up, down, ops.swiglu))
+    leaf = off.clone().requires_grad_(True)
+    out = moe_mlp(leaf, idx, w, gate_up, down, ops.swiglu)
+    (want,) = torch.autograd.grad(out, leaf, x[1:].view(T, H).clone(), retain_graph=True)
+    (got,) = torch.autograd.grad(out, leaf, x[1:].view(T, H))
+    assert torch.equal(got, want)
+    assert moe_gate(z, k, False, idx[:7])[0].shape == (7, k)  # as torch.gather does it
+    with pytest.raises((RuntimeError, ValueError, IndexError)):
+        moe_mlp(off.clone(), idx[:7], w[:7], gate_up, down, ops.swiglu)
+
+
 @pytest.mark.parametrize("E,k", [(8, 2), (33, 8), (128, 8), (300, 32)])
 @pytest.mark.parametrize("renorm", [True, False])
 @pytest.mark.parametrize("given", [False, True])

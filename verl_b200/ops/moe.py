@@ -165,7 +165,8 @@ def moe_gate(logits: torch.Tensor, k: int, renorm: bool, given: torch.Tensor | N
     """Softmax gate: (weights fp32 [T, k], experts int64 [T, k]) of the ``k`` most probable experts of every row of ``logits``
     [T, E], or of the ``given`` ones (router replay). ``renorm``: the weights are divided by their sum."""
     if (logits.is_cuda and logits.dtype in (torch.bfloat16, torch.float32) and logits.shape[1] <= 512 and k <= 32
-            and logits.stride(1) == 1 and (given is None or (given.dtype == torch.long and given.shape[1] == k))):
+            and logits.stride(1) == 1
+            and (given is None or (given.dtype == torch.long and given.is_cuda and given.shape == (logits.shape[0], k)))):
         if given is not None:
             given = given.contiguous()
         if torch.is_grad_enabled() and logits.requires_grad:
@@ -185,6 +186,7 @@ def _fused_mlp_ok(x, top_i, top_w, gate_up, down, swiglu) -> bool:
 
     H, I2 = x.shape[1], gate_up.shape[1]
     return (x.is_cuda and swiglu is nn.swiglu and x.shape[0] > 0 and x.dtype == gate_up.dtype == down.dtype == torch.bfloat16
+            and x.data_ptr() % 16 == 0 and top_i.shape == top_w.shape and top_i.shape[0] == x.shape[0]
             and top_i.dtype == torch.long and top_w.dtype == torch.float32 and gate_up.shape[0] <= 2048 and H % 64 == 0
             and I2 % 128 == 0 and gate_up.is_contiguous() and down.is_contiguous()
             and gate_up.data_ptr() % 16 == 0 and down.data_ptr() % 16 == 0)
@@ -229,6 +231,8 @@ class _RoutedMlpFn(torch.autograd.Function):
         (T, k), (P, H), (E, I2, _) = top_w.shape, xs.shape, gate_up.shape
         need_x, _, need_w, need_gu, need_down, _ = ctx.needs_input_grad
         stream, dy = _lib.stream(), dy.contiguous()
+        if dy.data_ptr() % 16:  # part of a larger gradient
+            dy = dy.clone()
         new = lambda *s: torch.empty(s, dtype=torch.bfloat16, device=dy.device)  # noqa: E731
 
         def weight_grad(weight, d, a):  # d^T a per expert
