@@ -401,6 +401,39 @@ def test_sampler_never_takes_a_token_of_no_weight():
     assert bool((tok == 77).all())
 
 
+@pytest.mark.parametrize("T,Hq,Hk,D,bs", [(1, 14, 2, 64, 16), (37, 28, 4, 128, 16), (5, 3, 1, 256, 8), (129, 9, 3, 64, 64)])
+@pytest.mark.parametrize("norm", [False, True])
+def test_head_norm_rope(T, Hq, Hk, D, bs, norm):
+    """Norms, positions and cache writes in one pass against the separate steps in fp64; rows without a slot are not written."""
+    from verl_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    full = torch.randn(T, (Hq + 2 * Hk) * D + 8, device="cuda", generator=gen).bfloat16()
+    src = full[:, 4 : 4 + (Hq + 2 * Hk) * D]
+    pos = torch.randint(0, 4096, (T,), device="cuda", generator=gen)
+    cos_t, sin_t = ops.rope_tables(D, 4096, 1e6, "cuda")
+    qw, kw = (1 + 0.1 * torch.randn(D, device="cuda", generator=gen).bfloat16() for _ in range(2))
+    NB = T // bs + 2
+    slots = torch.randperm(NB * bs, device="cuda", generator=gen)[:T]
+    slots[T // 2] = -1 if T > 1 else slots[0]
+    kc, vc = (torch.full((NB, Hk, bs, D), 9.0, device="cuda").bfloat16() for _ in range(2))
+    x = src.double().view(T, Hq + 2 * Hk, D)
+    if norm:
+        n = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6)
+        x = torch.cat([n[:, :Hq] * qw.double(), n[:, Hq : Hq + Hk] * kw.double(), x[:, Hq + Hk :]], 1)
+    c, s = cos_t[pos].double()[:, None], sin_t[pos].double()[:, None]
+    a, b = x[:, : Hq + Hk, : D // 2], x[:, : Hq + Hk, D // 2 :]
+    ref = torch.cat([torch.cat([a * c - b * s, b * c + a * s], -1), x[:, Hq + Hk :]], 1)
+    with torch.no_grad():
+        assert ops.head_norm_rope_(src, pos, cos_t, sin_t, Hq, Hk, D, (qw, kw) if norm else None, 1e-6, slots, kc, vc)
+    got = src.double().view(T, Hq + 2 * Hk, D)
+    assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * ref.abs().max()).all()  # one rounding to bf16, fp32 arithmetic
+    want_k, want_v = torch.full_like(kc, 9.0), torch.full_like(vc, 9.0)
+    k, v = (src[:, i : i + Hk * D].clone().view(T, Hk, D) for i in (Hq * D, (Hq + Hk) * D))  # that kernel takes 16-byte boundaries
+    ops.kv_cache_write(k, v, slots, want_k, want_v)
+    assert torch.equal(kc, want_k) and torch.equal(vc, want_v)
+
+
 @pytest.mark.parametrize("B,Hq,Hk,D,bs,maxlen", [(5, 28, 4, 128, 16, 700), (3, 4, 2, 64, 16, 300), (2, 32, 4, 128, 32, 3000),
                                                  (4, 40, 8, 128, 16, 150), (3, 32, 2, 128, 128, 1000),
                                                  (2, 8, 8, 128, 8, 260), (1, 14, 2, 64, 16, 110), (7, 8, 8, 64, 8, 129),

@@ -243,6 +243,28 @@ def rotate_pairs(x: torch.Tensor, positions: torch.Tensor, freqs: torch.Tensor, 
     return torch.cat((r, x[..., 2 * n :]), -1)
 
 
+def head_norm_rope_(qkv: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t: torch.Tensor, Hq: int, Hk: int, D: int,
+                    norms: tuple | None, eps: float, slots: torch.Tensor | None = None, k_cache: torch.Tensor | None = None,
+                    v_cache: torch.Tensor | None = None) -> bool:
+    """Serving, in place on packed ``qkv`` [T, (Hq + 2 Hk) * D]: RMS norm of every q and k head (``norms`` = weights [D] of q and of
+    k), rotate-half positions, and with ``slots`` the keys and values to the paged caches [NB, Hk, BS, D]; one kernel, one rounding.
+    False where it does not apply (nothing is done then): host tensors, gradients, other sizes, multimodal positions."""
+    if (not qkv.is_cuda or torch.is_grad_enabled() or qkv.dtype != torch.bfloat16 or D not in (64, 128, 256) or pos.dim() != 1
+            or pos.dtype != torch.long or qkv.dim() != 2 or qkv.stride(1) != 1 or qkv.stride(0) % 4 or qkv.data_ptr() % 8
+            or cos_t.shape[1] != D // 2 or not cos_t.is_contiguous() or not sin_t.is_contiguous()
+            or any(w.dtype != torch.bfloat16 or not w.is_contiguous() for w in norms or ())):
+        return False
+    if slots is not None and not (k_cache.dtype == v_cache.dtype == torch.bfloat16 and k_cache.is_contiguous() and v_cache.is_contiguous()
+                                  and (k_cache.data_ptr() | v_cache.data_ptr()) % 8 == 0):
+        return False
+    pos, (qw, kw) = pos.contiguous(), norms or (None, None)
+    rc = _lib.fn("vb_head_norm_rope")(qkv.data_ptr(), qkv.stride(0), pos.data_ptr(), cos_t.data_ptr(), sin_t.data_ptr(), _lib.ptr(qw),
+                                      _lib.ptr(kw), float(eps), qkv.shape[0], Hq, Hk, D, _lib.ptr(slots), _lib.ptr(k_cache),
+                                      _lib.ptr(v_cache), 0 if k_cache is None else k_cache.shape[2], _lib.stream())
+    _lib.check(rc, "vb_head_norm_rope")
+    return True
+
+
 def head_norm_rope_kv_write(qkv: torch.Tensor, q_weight: torch.Tensor | None, k_weight: torch.Tensor | None,
                             freqs: torch.Tensor | None, positions: torch.Tensor, slots: torch.Tensor, k_cache: torch.Tensor,
                             v_cache: torch.Tensor, heads: int, eps: float, *, interleaved: bool,

@@ -494,20 +494,31 @@ class NativeRolloutEngine:
         return bool(self.requests)
 
     # ------------------------------------------------------------ model pieces
-    def _layer_attn_in(self, layer, x, positions):
+    def _layer_attn_in(self, li, layer, x, positions, slots):
+        """Queries, keys and values of a layer; keys and values are in the cache at ``slots`` then."""
         c = self.cfg
         att = layer.self_attn
         qkv = self._mm(x, att.qkv_proj.weight, att.qkv_proj.bias)
         T = x.shape[0]
+        rope = self.model.rope(self.device)
+        norms = (att.q_norm.weight, att.k_norm.weight) if c.qk_norm else None
+        if ops.head_norm_rope_(qkv, positions, *rope, c.num_attention_heads, c.num_key_value_heads, c.head_dim, norms, c.rms_norm_eps,
+                               slots, self.k_cache[li], self.v_cache[li]):
+            return self._split_qkv(qkv)
         if c.qk_norm:
             q, k, v = qkv.split([c.q_size, c.kv_size, c.kv_size], dim=-1)
             q, _ = ops.rmsnorm(q.reshape(T * c.num_attention_heads, c.head_dim).contiguous(), att.q_norm.weight, c.rms_norm_eps)
             k, _ = ops.rmsnorm(k.reshape(T * c.num_key_value_heads, c.head_dim).contiguous(), att.k_norm.weight, c.rms_norm_eps)
             qkv = torch.cat([q.reshape(T, -1), k.reshape(T, -1), v], dim=-1)
-        rope = self.model.rope(self.device)
         qkv = ops.rope_qkv(qkv, positions, rope[0], rope[1], c.num_attention_heads, c.num_key_value_heads, c.head_dim,
                            mrope_section=c.mrope_section if positions.dim() == 2 else None,
                            mrope_interleaved=bool(getattr(c, "mrope_interleaved", False)))
+        q, k, v = self._split_qkv(qkv)
+        ops.kv_cache_write(k, v, slots, self.k_cache[li], self.v_cache[li])
+        return q, k, v
+
+    def _split_qkv(self, qkv):
+        c, T = self.cfg, qkv.shape[0]
         q = qkv[:, : c.q_size].view(T, c.num_attention_heads, c.head_dim)
         k = qkv[:, c.q_size : c.q_size + c.kv_size].view(T, c.num_key_value_heads, c.head_dim)
         v = qkv[:, c.q_size + c.kv_size :].view(T, c.num_key_value_heads, c.head_dim)
@@ -645,8 +656,7 @@ class NativeRolloutEngine:
         h = ops.embedding(ids, self.model.embed_tokens.weight)
 
         def attend(li, layer, x):
-            q, k, v = self._layer_attn_in(layer, x, positions)
-            ops.kv_cache_write(k, v, slots, self.k_cache[li], self.v_cache[li])
+            q, k, v = self._layer_attn_in(li, layer, x, positions, slots)
             return ops.paged_decode_attention(q, self.k_cache[li], self.v_cache[li], block_table, seq_lens,
                                               num_splits=splits, work=work)
 
@@ -842,8 +852,7 @@ class NativeRolloutEngine:
                 inject = {li: (rows_all, torch.cat([v[li] for v in ds_vals])) for li in range(len(ds_vals[0]))}
 
         def attend(li, layer, x):
-            q, k, v = self._layer_attn_in(layer, x, pos)
-            ops.kv_cache_write(k, v, slots, self.k_cache[li], self.v_cache[li])
+            q, k, v = self._layer_attn_in(li, layer, x, pos, slots)
             if not has_ctx:
                 return ops.attention_varlen(q, k, v, cu_q, max_q, causal=True)
             k_all = torch.cat([self.k_cache[li][blk, :, off], k], dim=0)[order_t]
