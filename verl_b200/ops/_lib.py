@@ -14,9 +14,12 @@ from ctypes import c_float, c_int, c_longlong, c_ulonglong, c_void_p
 from pathlib import Path
 
 import torch
+from torch.autograd import forward_ad as _forward_ad
 
 _LIB = None
 _LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libverl_b200.so"
+
+_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
 
 P, I, L, F, U = c_void_p, c_int, c_longlong, c_float, c_ulonglong
 
@@ -160,12 +163,17 @@ def available() -> bool:
         return False
 
 
+_FNS: dict = {}
+
+
 def fn(name: str):
-    lib = load()
-    try:
-        return getattr(lib, name)
-    except AttributeError as e:
-        raise NativeLibraryError(f"symbol {name} not in {_LIB_PATH}; rebuild the native library") from e
+    f = _FNS.get(name)
+    if f is None:
+        try:
+            f = _FNS[name] = getattr(load(), name)
+        except AttributeError as e:
+            raise NativeLibraryError(f"symbol {name} not in {_LIB_PATH}; rebuild the native library") from e
+    return f
 
 
 def set_pdl(on: bool) -> None:
@@ -183,7 +191,15 @@ def ptr(t) -> int | None:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device, without the stream object that ``torch.cuda.current_stream`` builds (7 us a call,
+    a fifth of the host time of a forward on short sequences; 0.3 us this way)."""
+    return _raw_stream(_current_device())
+
+
+def plain() -> bool:
+    """Nothing records what is computed: no gradients, no forward-mode level. An autograd function's forward is then its result, and
+    going through ``Function.apply`` only costs (5 us a call)."""
+    return not torch.is_grad_enabled() and _forward_ad._current_level < 0
 
 
 def check(rc: int, what: str) -> None:

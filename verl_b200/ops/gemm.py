@@ -159,4 +159,7 @@ class _LinearFn(torch.autograd.Function):
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
+    if _lib.plain():
+        y = gemm(x if x.dim() == 2 else x.reshape(-1, x.shape[-1]), weight, bias=bias, out_dtype=x.dtype)
+        return y if x.dim() == 2 else y.view(*x.shape[:-1], weight.shape[0])
     return _LinearFn.apply(x, weight, bias)

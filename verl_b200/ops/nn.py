@@ -22,22 +22,22 @@ class _RMSNormFn(torch.autograd.Function):
     """y = rmsnorm(x + residual) * w; also returns the new residual stream (x + residual)."""
 
     @staticmethod
-    def forward(ctx, x, residual, weight, eps):
+    def _run(x, residual, weight, eps):
         H = x.shape[-1]
         x2 = x.reshape(-1, H)
         rows = x2.shape[0]
         y = torch.empty_like(x2)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-        if residual is not None:
-            r2 = residual.reshape(-1, H)
-            h = torch.empty_like(x2)
-            rc = _lib.fn("vb_rmsnorm_fwd")(x2.data_ptr(), r2.data_ptr(), weight.data_ptr(), y.data_ptr(), h.data_ptr(),
-                                           rstd.data_ptr(), rows, H, eps, _lib.stream())
-        else:
-            h = x2
-            rc = _lib.fn("vb_rmsnorm_fwd")(x2.data_ptr(), None, weight.data_ptr(), y.data_ptr(), None,
-                                           rstd.data_ptr(), rows, H, eps, _lib.stream())
+        r2 = None if residual is None else residual.reshape(-1, H)
+        h = x2 if residual is None else torch.empty_like(x2)
+        rc = _lib.fn("vb_rmsnorm_fwd")(x2.data_ptr(), _lib.ptr(r2), weight.data_ptr(), y.data_ptr(),
+                                       None if residual is None else h.data_ptr(), rstd.data_ptr(), rows, H, eps, _lib.stream())
         _lib.check(rc, "vb_rmsnorm_fwd")
+        return y, h, rstd
+
+    @staticmethod
+    def forward(ctx, x, residual, weight, eps):
+        y, h, rstd = _RMSNormFn._run(x, residual, weight, eps)
         ctx.save_for_backward(h, weight, rstd)
         ctx.has_res = residual is not None
         ctx.shape = x.shape
@@ -73,9 +73,11 @@ class _RMSNormFn(torch.autograd.Function):
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, residual: torch.Tensor | None = None):
     """Returns ``(normed, new_residual)`` where ``new_residual = x + residual`` (or ``x``)."""
     if x.is_cuda:
-        if residual is None and not torch.is_grad_enabled():
-            pass
-        return _RMSNormFn.apply(x.contiguous(), None if residual is None else residual.contiguous(), weight, eps)
+        x, residual = x.contiguous(), None if residual is None else residual.contiguous()
+        if _lib.plain():
+            y, h, _ = _RMSNormFn._run(x, residual, weight, eps)
+            return y.reshape(x.shape), x if residual is None else h.reshape(x.shape)
+        return _RMSNormFn.apply(x, residual, weight, eps)
     h = x if residual is None else x + residual
     return _rmsnorm_ref(h, weight, eps), h
 
@@ -187,8 +189,11 @@ def rope_qkv(qkv: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t: t
         mrope_section = None
     if qkv.is_cuda and (mrope_section is None or
                         (not mrope_interleaved and all(int(x) % 8 == 0 for x in mrope_section[:2]))):
-        return _RopeFn.apply(qkv, pos.contiguous(), cos_t, sin_t, Hq, Hk, D,
-                             None if mrope_section is None else tuple(int(x) for x in mrope_section))
+        pos, sections = pos.contiguous(), None if mrope_section is None else tuple(int(x) for x in mrope_section)
+        if _lib.plain():
+            _RopeFn._run(qkv, pos, cos_t, sin_t, Hq, Hk, D, sections, 0)
+            return qkv
+        return _RopeFn.apply(qkv, pos, cos_t, sin_t, Hq, Hk, D, sections)
     if mrope_section is not None:
         c, s_ = _mrope_cos_sin(pos, cos_t, sin_t, mrope_section, mrope_interleaved)
         q = _rope_apply(qkv[:, : Hq * D], c, s_, Hq, D)
@@ -211,13 +216,17 @@ def _rope_apply(t, c, s_, n_heads, D):
 # ---------------------------------------------------------------------------- SwiGLU
 class _SwiGLUFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, gu):
+    def _run(gu):
         T, I2 = gu.shape
         out = torch.empty(T, I2 // 2, dtype=gu.dtype, device=gu.device)
         rc = _lib.fn("vb_swiglu_fwd")(gu.data_ptr(), out.data_ptr(), T, I2 // 2, None, _lib.stream())
         _lib.check(rc, "vb_swiglu_fwd")
-        ctx.save_for_backward(gu)
         return out
+
+    @staticmethod
+    def forward(ctx, gu):
+        ctx.save_for_backward(gu)
+        return _SwiGLUFn._run(gu)
 
     @staticmethod
     def backward(ctx, dout):
@@ -234,7 +243,7 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     """``silu(gate) * up`` for ``gate_up = [gate | up]`` along the last dim."""
     if gate_up.is_cuda:
         shape = gate_up.shape
-        out = _SwiGLUFn.apply(gate_up.reshape(-1, shape[-1]).contiguous())
+        out = (_SwiGLUFn._run if _lib.plain() else _SwiGLUFn.apply)(gate_up.reshape(-1, shape[-1]).contiguous())
         return out.reshape(*shape[:-1], shape[-1] // 2)
     g, u = gate_up.chunk(2, dim=-1)
     return F.silu(g) * u

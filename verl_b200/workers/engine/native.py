@@ -626,6 +626,9 @@ class NativeEngine(BaseEngine):
         qkv = (c.num_attention_heads + 2 * c.num_key_value_heads) * c.head_dim
         per_token = 2 * (5 * c.hidden_size + qkv + c.num_attention_heads * c.head_dim + 3 * c.intermediate_size) + 64
         per_layer = int(tokens * per_token * 1.1)
+        if n_layers * per_layer <= 1 << 28:  # 256 MB: kept without asking what is free, which takes 1.6 ms of a small micro-batch's 10
+            self.last_kept_layers = n_layers
+            return n_layers
         free, total = torch.cuda.mem_get_info(self.device)
         free += torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
         reserve = max(12 << 30, total // 12) + 2 * per_layer
