@@ -65,6 +65,17 @@ def test_gemm_few_rows(M, N, K):
     assert ((got - want).abs() <= bound + 2.0 ** -8 * want.abs() + 2.0 ** -23).all()
 
 
+@pytest.mark.parametrize("T,N", [(1, 2), (7, 34), (8, 512), (511, 514), (512, 1026), (3000, 4608), (5, 33)])
+def test_colsum(T, N):
+    from verl_b200.ops.gemm import colsum
+
+    torch.manual_seed(T)
+    x = torch.randn(T, N + 2, device="cuda").bfloat16()[:, :N]
+    ref = x.double().sum(0)
+    bound = x.double().abs().sum(0) * T * 2.0 ** -24 + 2.0 ** -8 * ref.abs()  # an fp32 sum of T terms, one rounding to bf16
+    assert ((colsum(x).double() - ref).abs() <= bound).all()
+
+
 def test_gemm_fp32_accumulate_and_bias():
     from verl_b200.ops import gemm
 

@@ -36,6 +36,8 @@ _SIGS = {
     "vb_lmhead_dlogits": ([P, P, P, I, I, I, I, F, P, P, P, P, P, L, P, P], I),
     # elementwise
     "vb_rmsnorm_fwd": ([P, P, P, P, P, P, L, I, F, P], I),
+    "vb_colsum_parts": ([I], I),
+    "vb_colsum_bf16": ([P, L, I, I, P, P, P], I),
     "vb_rmsnorm_bwd_parts": ([L], I),
     "vb_rmsnorm_bwd": ([P, P, P, P, P, P, P, P, I, L, I, P], I),
     "vb_head_norm_rope": ([P, L, P, P, P, P, P, F, L, I, I, I, P, P, P, I, P], I),

@@ -124,6 +124,18 @@ def _splitk_workspace(device, stream):
     return got
 
 
+def colsum(x: torch.Tensor) -> torch.Tensor:
+    """Sum over the rows of ``x`` [T, N], in fp32, in its dtype."""
+    T, N = x.shape
+    if not x.is_cuda or x.dtype != torch.bfloat16 or N % 2 or x.stride(1) != 1 or x.stride(0) % 2 or x.data_ptr() % 4 or T == 0 or N == 0:
+        return x.float().sum(0).to(x.dtype)
+    out = torch.empty(N, dtype=x.dtype, device=x.device)
+    work = torch.empty((_lib.fn("vb_colsum_parts")(T), N), dtype=torch.float32, device=x.device)
+    rc = _lib.fn("vb_colsum_bf16")(x.data_ptr(), x.stride(0), T, N, work.data_ptr(), out.data_ptr(), _lib.stream())
+    _lib.check(rc, "vb_colsum_bf16")
+    return out
+
+
 class _LinearFn(torch.autograd.Function):
     """y = x W^T (+ b). If ``weight.main_grad`` exists (fp32, same shape) the weight gradient
     is accumulated into it by the GEMM epilogue and autograd sees ``None`` for the weight."""
@@ -154,7 +166,7 @@ class _LinearFn(torch.autograd.Function):
             else:
                 dw = gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=weight.dtype)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy2.float().sum(0).to(dy.dtype)
+            db = colsum(dy2)
         return dx, dw, db
 
 
