@@ -438,11 +438,53 @@ def test_head_norm_rope(T, Hq, Hk, D, bs, norm):
     with torch.no_grad():
         assert ops.head_norm_rope_(src, pos, cos_t, sin_t, Hq, Hk, D, (qw, kw) if norm else None, 1e-6, slots, kc, vc)
     got = src.double().view(T, Hq + 2 * Hk, D)
-    assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * ref.abs().max()).all()  # one rounding to bf16, fp32 arithmetic
+    # roundings to bf16 of the normed head, carried by the rotation, and of the result, 2^-8 each
+    size = torch.cat([(a.abs() + b.abs()).repeat(1, 1, 2), x[:, Hq + Hk :].abs()], 1)
+    assert ((got - ref).abs() <= 2.0 ** -7 * size + 1e-5 * ref.abs().max()).all()
     want_k, want_v = torch.full_like(kc, 9.0), torch.full_like(vc, 9.0)
     k, v = (src[:, i : i + Hk * D].clone().view(T, Hk, D) for i in (Hq * D, (Hq + Hk) * D))  # that kernel takes 16-byte boundaries
     ops.kv_cache_write(k, v, slots, want_k, want_v)
     assert torch.equal(kc, want_k) and torch.equal(vc, want_v)
+
+
+@pytest.mark.parametrize("T,Hq,Hk,D", [(1, 14, 2, 64), (300, 7, 1, 128), (33, 4, 4, 256), (2000, 8, 2, 64)])
+@pytest.mark.parametrize("norm", [False, True])
+def test_qkv_heads_gradients(T, Hq, Hk, D, norm):
+    """Forward as without gradients, bit for bit; gradients of the projection and of the norms against fp64, added to ``main_grad``."""
+    from verl_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()  # noqa: E731
+    qkv = rnd(T, (Hq + 2 * Hk) * D).requires_grad_(True)
+    pos = torch.randint(0, 4096, (T,), device="cuda", generator=gen)
+    cos_t, sin_t = ops.rope_tables(D, 4096, 1e6, "cuda")
+    w = [(1 + 0.1 * rnd(D)).requires_grad_(True) for _ in range(2)]
+    w[1].main_grad = torch.full((D,), 2.0, device="cuda")
+    grads = [rnd(T, n, D) for n in (Hq, Hk, Hk)]
+    got = ops.qkv_heads(qkv, pos, cos_t, sin_t, Hq, Hk, D, tuple(w) if norm else None, 1e-6)
+    with torch.no_grad():
+        plain = ops.qkv_heads(qkv.detach().clone(), pos, cos_t, sin_t, Hq, Hk, D, tuple(w) if norm else None, 1e-6)
+    assert all(torch.equal(g, p) for g, p in zip(got, plain))
+    if not norm:
+        with torch.no_grad():
+            assert torch.equal(torch.cat(got, 1).view(T, -1), ops.rope_qkv(qkv.detach().clone(), pos, cos_t, sin_t, Hq, Hk, D))
+    torch.autograd.backward(got, grads)
+    x, (qw, kw) = qkv.detach().double().requires_grad_(True), (t.detach().double().requires_grad_(True) for t in w)
+    h = x.view(T, Hq + 2 * Hk, D)
+    if norm:
+        n = h * torch.rsqrt(h.pow(2).mean(-1, keepdim=True) + 1e-6)
+        h = torch.cat([n[:, :Hq] * qw, n[:, Hq : Hq + Hk] * kw, h[:, Hq + Hk :]], 1)
+    c, s = cos_t[pos].double()[:, None], sin_t[pos].double()[:, None]
+    a, b = h[:, : Hq + Hk, : D // 2], h[:, : Hq + Hk, D // 2 :]
+    y = torch.cat([torch.cat([a * c - b * s, b * c + a * s], -1), h[:, Hq + Hk :]], 1)
+    y.backward(torch.cat(grads, 1).double())
+    # the rotated gradient and the result are rounded, 2^-8 each; the norm's weights and 1 / rms carry the first one by less than 2
+    _bf16_close(qkv.grad, x.grad, ulps=3)
+    if norm:
+        for g, ref, heads in ((w[0].grad.double(), qw.grad, Hq), (w[1].main_grad.double() - 2.0, kw.grad, Hk)):
+            # T * heads terms of about 1, their gradient factor rounded (2^-8, of either sign: 6 sigma), and the result in bf16
+            bound = 2.0 ** -8 * 6 * (T * heads) ** 0.5 + 2.0 ** -8 * ref.abs()
+            assert ((g - ref).abs() <= bound).all()
 
 
 @pytest.mark.parametrize("B,Hq,Hk,D,bs,maxlen", [(5, 28, 4, 128, 16, 700), (3, 4, 2, 64, 16, 300), (2, 32, 4, 128, 32, 3000),

@@ -222,31 +222,18 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __rest
   }
 }
 
-// Serving: what lies between a layer's projection and its attention, in one pass over packed rows qkv [T, (Hq + 2 Hk) D]. RMS norm of
-// every q and k head (weights [D] shared by the heads; null: none) and rotate-half positions, in place, in fp32 up to one rounding; k
-// and v also to their places in the paged caches [num_blocks, Hk, block_size, D] (slots null: no cache; slot < 0: no write).
-// D / 8 lanes per head, each with four elements of both halves. Bound by latency in a decode step, by its bytes in a prefill. It took
-// the place of a rotation and a cache write, with norms also of two copies, two norms and a concatenation: a decode step of 24
-// sequences, 32 / 4 heads with norms: 16 us a layer in seven launches, 3 in one.
+// What lies between a layer's projection and its attention, in one pass over packed rows qkv [T, (Hq + 2 Hk) D]: RMS norm of every q
+// and k head (weights [D] shared by the heads; null: none; rounded to bf16, as a norm of its own is), rotate-half positions, to `out`
+// (may be qkv); k and v also to their places in the paged caches [num_blocks, Hk, block_size, D] (slots null: no cache; slot < 0: no
+// write). D / 8 lanes per head, each with four elements of both halves. Bound by latency in a decode step, by its bytes in a prefill or
+// in training. It took the place of a rotation and a cache write, with norms also of two copies, two norms and a concatenation: a decode
+// step of 24 sequences, 32 / 4 heads with norms: 16 us a layer in seven launches, 3 in one; a forward on 6400
+// such tokens 490 us a layer, 122 in one.
 template <int D>
-__global__ void __launch_bounds__(256) head_norm_rope_kernel(
-    __nv_bfloat16* qkv, long long stride, const long long* pos, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-    const __nv_bfloat16* __restrict__ qw, const __nv_bfloat16* __restrict__ kw, float eps, long long T, int Hq, int Hk,
-    const long long* slots, __nv_bfloat16* kc, __nv_bfloat16* vc, int block_size) {
-  constexpr int LPH = D / 8, HALF = D / 2;
-  pdl_trigger();
-  pdl_wait();
-  const int heads = Hq + Hk + (slots ? Hk : 0);
-  const long long unit = ((long long)blockIdx.x * 256 + threadIdx.x) / LPH;
-  const int sub = threadIdx.x % LPH;
-  if (unit - threadIdx.x % 32 / LPH >= T * heads) return;  // whole warps: the lanes of a norm stay together
-  const bool in = unit < T * heads;
-  const long long t = in ? unit / heads : 0;
-  const int h = in ? (int)(unit % heads) : 0;
-  __nv_bfloat16* x = qkv + t * stride + (long long)h * D + sub * 4;
-  uint2 ra = *reinterpret_cast<const uint2*>(x), rb = *reinterpret_cast<const uint2*>(x + HALF);
+struct HeadPart {  // a lane's share of a head
   float a[4], b[4];
-  {
+  __device__ __forceinline__ void load(const __nv_bfloat16* x) {
+    const uint2 ra = *reinterpret_cast<const uint2*>(x), rb = *reinterpret_cast<const uint2*>(x + D / 2);
     const __nv_bfloat162 *pa = reinterpret_cast<const __nv_bfloat162*>(&ra), *pb = reinterpret_cast<const __nv_bfloat162*>(&rb);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -254,46 +241,151 @@ __global__ void __launch_bounds__(256) head_norm_rope_kernel(
       a[2 * i] = fa.x, a[2 * i + 1] = fa.y, b[2 * i] = fb.x, b[2 * i + 1] = fb.y;
     }
   }
+  __device__ __forceinline__ void store(__nv_bfloat16* x) const {
+    *reinterpret_cast<uint2*>(x) = make_uint2(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]));
+    *reinterpret_cast<uint2*>(x + D / 2) = make_uint2(pack_bf16x2(b[0], b[1]), pack_bf16x2(b[2], b[3]));
+  }
+  __device__ __forceinline__ void round() {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      a[i] = __bfloat162float(__float2bfloat16(a[i]));
+      b[i] = __bfloat162float(__float2bfloat16(b[i]));
+    }
+  }
+  // by the angles at the token's position; sign -1: back
+  __device__ __forceinline__ void rotate(const float* cos_t, const float* sin_t, float sign) {
+    const float4 c = *reinterpret_cast<const float4*>(cos_t), s = *reinterpret_cast<const float4*>(sin_t);
+    const float cs[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x * sign, s.y * sign, s.z * sign, s.w * sign};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float x = a[i], y = b[i];
+      a[i] = __fmaf_rn(x, cs[i], -__fmul_rn(y, sn[i]));  // as rope_kernel comes out, bit for bit
+      b[i] = __fmaf_rn(y, cs[i], __fmul_rn(x, sn[i]));
+    }
+  }
+  // sum over the head of a * p.a + b * p.b; the D / 8 lanes of a head call it together
+  __device__ __forceinline__ float dot(const HeadPart& p) const {
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s += a[i] * p.a[i] + b[i] * p.b[i];
+#pragma unroll
+    for (int o = 1; o < D / 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+  }
+};
+
+template <int D>
+__global__ void __launch_bounds__(256) head_norm_rope_kernel(
+    const __nv_bfloat16* qkv, long long stride, __nv_bfloat16* out, long long out_stride, const long long* pos,
+    const float* __restrict__ cos_t, const float* __restrict__ sin_t, const __nv_bfloat16* __restrict__ qw,
+    const __nv_bfloat16* __restrict__ kw, float eps, long long T, int Hq, int Hk, const long long* slots, __nv_bfloat16* kc,
+    __nv_bfloat16* vc, int block_size) {
+  constexpr int LPH = D / 8, HALF = D / 2;
+  pdl_trigger();
+  pdl_wait();
+  const int heads = Hq + Hk + (slots || out != qkv ? Hk : 0);
+  const long long unit = ((long long)blockIdx.x * 256 + threadIdx.x) / LPH;
+  const int sub = threadIdx.x % LPH;
+  if (unit - threadIdx.x % 32 / LPH >= T * heads) return;  // whole warps: the lanes of a norm stay together
+  const bool in = unit < T * heads;
+  const long long t = in ? unit / heads : 0;
+  const int h = in ? (int)(unit % heads) : 0;
+  HeadPart<D> x;
+  x.load(qkv + t * stride + (long long)h * D + sub * 4);
   if (qw != nullptr) {
-    float ss = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) ss += a[i] * a[i] + b[i] * b[i];
-#pragma unroll
-    for (int o = 1; o < LPH; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float rs = rsqrtf(x.dot(x) / D + eps);
     if (h < Hq + Hk) {
-      const float rs = rsqrtf(ss / D + eps);
-      const __nv_bfloat16* w = (h < Hq ? qw : kw) + sub * 4;
+      HeadPart<D> w;
+      w.load((h < Hq ? qw : kw) + sub * 4);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        a[i] *= rs * __bfloat162float(w[i]);
-        b[i] *= rs * __bfloat162float(w[HALF + i]);
+        x.a[i] = x.a[i] * rs * w.a[i];
+        x.b[i] = x.b[i] * rs * w.b[i];
       }
+      x.round();
     }
   }
   if (!in) return;
-  if (h < Hq + Hk) {
-    const long long at = pos[t] * HALF + sub * 4;
-    const float4 c = *reinterpret_cast<const float4*>(cos_t + at), s = *reinterpret_cast<const float4*>(sin_t + at);
-    const float cs[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x, s.y, s.z, s.w};
-    float oa[4], ob[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      oa[i] = a[i] * cs[i] - b[i] * sn[i];
-      ob[i] = b[i] * cs[i] + a[i] * sn[i];
-    }
-    ra = make_uint2(pack_bf16x2(oa[0], oa[1]), pack_bf16x2(oa[2], oa[3]));
-    rb = make_uint2(pack_bf16x2(ob[0], ob[1]), pack_bf16x2(ob[2], ob[3]));
-    *reinterpret_cast<uint2*>(x) = ra;
-    *reinterpret_cast<uint2*>(x + HALF) = rb;
-  }
+  if (h < Hq + Hk) x.rotate(cos_t + pos[t] * HALF + sub * 4, sin_t + pos[t] * HALF + sub * 4, 1.f);
+  if (h < Hq + Hk || out != qkv) x.store(out + t * out_stride + (long long)h * D + sub * 4);
   if (slots != nullptr && h >= Hq) {
     const long long slot = slots[t];
     if (slot < 0) return;
     const bool key = h < Hq + Hk;
     const long long row = (slot / block_size * Hk + (h - Hq - (key ? 0 : Hk))) * block_size + slot % block_size;
-    __nv_bfloat16* dst = (key ? kc : vc) + row * D + sub * 4;
-    *reinterpret_cast<uint2*>(dst) = ra;
-    *reinterpret_cast<uint2*>(dst + HALF) = rb;
+    x.store((key ? kc : vc) + row * D + sub * 4);
+  }
+}
+
+// Gradient of the projection from those of q [T, Hq D], k and v [T, Hk D]: rotation back (rounded, as a rotation of its own is), norm,
+// and the sums of the norms' weights per block, part [2][gridDim.x][D] (with norms). x: the projection (with norms). One pass in place
+// of three zero-filled buffers, their sum, a copy, a rotation and two norms.
+template <int D>
+__global__ void __launch_bounds__(256) head_norm_rope_bwd_kernel(
+    const __nv_bfloat16* __restrict__ dq, const __nv_bfloat16* __restrict__ dk, const __nv_bfloat16* __restrict__ dv,
+    const __nv_bfloat16* __restrict__ x, long long x_stride, const long long* __restrict__ pos, const float* __restrict__ cos_t,
+    const float* __restrict__ sin_t, const __nv_bfloat16* __restrict__ qw, const __nv_bfloat16* __restrict__ kw, float eps, long long T,
+    int Hq, int Hk, __nv_bfloat16* __restrict__ dqkv, float* __restrict__ part) {
+  constexpr int LPH = D / 8, HALF = D / 2, GROUPS = 256 / LPH;
+  __shared__ float sums[2][GROUPS][D];
+  const int heads = Hq + 2 * Hk, sub = threadIdx.x % LPH, group = threadIdx.x / LPH;
+  const long long total = T * heads;
+  HeadPart<D> sq{}, sk{};
+  for (long long u0 = (long long)blockIdx.x * GROUPS; u0 < total; u0 += (long long)gridDim.x * GROUPS) {
+    const bool in = u0 + group < total;
+    const long long unit = in ? u0 + group : 0, t = unit / heads;
+    const int h = (int)(unit % heads);
+    const __nv_bfloat16* from = h < Hq ? dq + (t * Hq + h) * D : h < Hq + Hk ? dk + (t * Hk + h - Hq) * D : dv + (t * Hk + h - Hq - Hk) * D;
+    HeadPart<D> d;
+    d.load(from + sub * 4);
+    if (h < Hq + Hk) {
+      d.rotate(cos_t + pos[t] * HALF + sub * 4, sin_t + pos[t] * HALF + sub * 4, -1.f);
+      d.round();
+    }
+    if (qw != nullptr) {
+      HeadPart<D> y, w;
+      y.load(x + t * x_stride + (long long)h * D + sub * 4);
+      w.load((h < Hq ? qw : kw) + sub * 4);
+      const float rs = rsqrtf(y.dot(y) / D + eps);
+      HeadPart<D> g;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        y.a[i] *= rs;
+        y.b[i] *= rs;
+        g.a[i] = d.a[i] * w.a[i];
+        g.b[i] = d.b[i] * w.b[i];
+      }
+      const float mean = g.dot(y) / D;
+      if (in && h < Hq + Hk) {
+        const float to_q = h < Hq ? 1.f : 0.f, to_k = 1.f - to_q;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float pa = d.a[i] * y.a[i], pb = d.b[i] * y.b[i];
+          sq.a[i] = fmaf(to_q, pa, sq.a[i]);
+          sq.b[i] = fmaf(to_q, pb, sq.b[i]);
+          sk.a[i] = fmaf(to_k, pa, sk.a[i]);
+          sk.b[i] = fmaf(to_k, pb, sk.b[i]);
+          d.a[i] = rs * (g.a[i] - y.a[i] * mean);
+          d.b[i] = rs * (g.b[i] - y.b[i] * mean);
+        }
+      }
+    }
+    if (in) d.store(dqkv + unit * D + sub * 4);
+  }
+  if (qw == nullptr) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    sums[0][group][sub * 4 + i] = sq.a[i];
+    sums[0][group][HALF + sub * 4 + i] = sq.b[i];
+    sums[1][group][sub * 4 + i] = sk.a[i];
+    sums[1][group][HALF + sub * 4 + i] = sk.b[i];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * D; i += 256) {
+    float s = 0.f;
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) s += sums[i / D][g][i % D];
+    part[((long long)(i / D) * gridDim.x + blockIdx.x) * D + i % D] = s;
   }
 }
 
@@ -502,21 +594,22 @@ extern "C" int vb_rope(void* q, void* k, long long q_stride, long long k_stride,
   return rope_launch(q, k, q_stride, k_stride, pos, cos_t, sin_t, T, Hq, Hk, D, backward, 0, 0, stream);
 }
 
-// D 64, 128 or 256; rows and caches on 8-byte boundaries. qw and kw both or neither.
-extern "C" int vb_head_norm_rope(void* qkv, long long stride, const long long* pos, const float* cos_t, const float* sin_t, const void* qw,
-                                 const void* kw, float eps, long long T, int Hq, int Hk, int D, const long long* slots, void* kc, void* vc,
-                                 int block_size, cudaStream_t stream) {
+// D 64, 128 or 256; rows, results and caches on 8-byte boundaries. qw and kw both or neither.
+extern "C" int vb_head_norm_rope(const void* qkv, long long stride, void* out, long long out_stride, const long long* pos,
+                                 const float* cos_t, const float* sin_t, const void* qw, const void* kw, float eps, long long T, int Hq,
+                                 int Hk, int D, const long long* slots, void* kc, void* vc, int block_size, cudaStream_t stream) {
   if (T <= 0) return 0;
-  if ((stride & 3) || (reinterpret_cast<uintptr_t>(qkv) & 7) || (qw == nullptr) != (kw == nullptr) ||
+  if (((stride | out_stride) & 3) || ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 7) ||
+      (qw == nullptr) != (kw == nullptr) ||
       (slots && (((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 7) || block_size <= 0)))
     return -3;
-  const long long threads = T * (Hq + Hk + (slots ? Hk : 0)) * (D / 8), blocks = (threads + 255) / 256;
+  const long long threads = T * (Hq + Hk + (slots || out != qkv ? Hk : 0)) * (D / 8), blocks = (threads + 255) / 256;
   if (blocks > 0x7fffffffLL) return -3;
   cudaError_t e;
 #define VB_HNR(DD)                                                                                                                  \
-  e = vb_launch_pdl(head_norm_rope_kernel<DD>, dim3((unsigned)blocks), dim3(256), 0, stream, 1, (__nv_bfloat16*)qkv, stride, pos, cos_t, \
-                    sin_t, (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, eps, T, Hq, Hk, slots, (__nv_bfloat16*)kc,             \
-                    (__nv_bfloat16*)vc, block_size)
+  e = vb_launch_pdl(head_norm_rope_kernel<DD>, dim3((unsigned)blocks), dim3(256), 0, stream, 1, (const __nv_bfloat16*)qkv, stride,    \
+                    (__nv_bfloat16*)out, out_stride, pos, cos_t, sin_t, (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, eps, T, Hq, \
+                    Hk, slots, (__nv_bfloat16*)kc, (__nv_bfloat16*)vc, block_size)
   if (D == 64) VB_HNR(64);
   else if (D == 128) VB_HNR(128);
   else if (D == 256) VB_HNR(256);
@@ -524,6 +617,36 @@ extern "C" int vb_head_norm_rope(void* qkv, long long stride, const long long* p
 #undef VB_HNR
   vb_count_launch();
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+// dq, dk, dv, dqkv contiguous and on 8-byte boundaries. With norms: x the projection, part fp32 [2, parts, D], dqw and dkw fp32 [D]
+// (accumulate: added to).
+extern "C" int vb_head_norm_rope_bwd_parts() { return 4 * vb_num_sms(); }
+extern "C" int vb_head_norm_rope_bwd(const void* dq, const void* dk, const void* dv, const void* x, long long x_stride,
+                                     const long long* pos, const float* cos_t, const float* sin_t, const void* qw, const void* kw,
+                                     float eps, long long T, int Hq, int Hk, int D, void* dqkv, float* part, float* dqw, float* dkw,
+                                     int accumulate_q, int accumulate_k, cudaStream_t stream) {
+  if (T <= 0) return 0;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv) |
+                       reinterpret_cast<uintptr_t>(dqkv) | (qw ? reinterpret_cast<uintptr_t>(x) : 0);
+  if ((at & 7) || (qw && ((x_stride & 3) || !kw || !part || !dqw || !dkw))) return -3;
+  const int parts = vb_head_norm_rope_bwd_parts();
+#define VB_HNRB(DD)                                                                                                                \
+  head_norm_rope_bwd_kernel<DD><<<parts, 256, 0, stream>>>((const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, \
+                                                           (const __nv_bfloat16*)x, x_stride, pos, cos_t, sin_t,                    \
+                                                           (const __nv_bfloat16*)qw, (const __nv_bfloat16*)kw, eps, T, Hq, Hk,      \
+                                                           (__nv_bfloat16*)dqkv, part)
+  if (D == 64) VB_HNRB(64);
+  else if (D == 128) VB_HNRB(128);
+  else if (D == 256) VB_HNRB(256);
+  else return -3;
+#undef VB_HNRB
+  if (qw) {
+    colsum_kernel<float><<<(D + 31) / 32, 1024, 0, stream>>>(part, parts, D, dqw, accumulate_q);
+    colsum_kernel<float><<<(D + 31) / 32, 1024, 0, stream>>>(part + (long long)parts * D, parts, D, dkw, accumulate_k);
+  }
+  vb_count_launch(qw ? 3 : 1);
+  return (int)cudaGetLastError();
 }
 
 // Multimodal RoPE: pos is [3, T]; s0 / s1 = number of rotary frequencies (of D / 2) that follow the temporal / height

@@ -308,19 +308,23 @@ class Attention(nn.Module):
 
             x = copy_to_tp_region(x, self.tp_group)
         qkv = self.qkv_proj(x)
+        norms = None
         if cfg.qk_norm:
-            q, k, v = qkv.split([cfg.q_size, cfg.kv_size, cfg.kv_size], dim=-1)
-            qw, kw = self.q_norm.weight, self.k_norm.weight
+            norms = self.q_norm.weight, self.k_norm.weight
             if self.tp_group is not None:  # shared by all heads: every rank sees its own heads' share of the gradient
-                qw, kw = copy_to_tp_region(qw, self.tp_group), copy_to_tp_region(kw, self.tp_group)
-            q, _ = ops.rmsnorm(q.reshape(T * Hq, D), qw, cfg.rms_norm_eps)
-            k, _ = ops.rmsnorm(k.reshape(T * Hk, D), kw, cfg.rms_norm_eps)
-            qkv = torch.cat([q.reshape(T, -1), k.reshape(T, -1), v], dim=-1)
-        qkv = ops.rope_qkv(qkv, batch.position_ids, rope[0], rope[1], Hq, Hk, D, mrope_section=cfg.mrope_section,
-                           mrope_interleaved=cfg.mrope_interleaved)
-        q = qkv[:, : cfg.q_size].view(T, Hq, D)
-        k = qkv[:, cfg.q_size : cfg.q_size + cfg.kv_size].view(T, Hk, D)
-        v = qkv[:, cfg.q_size + cfg.kv_size :].view(T, Hk, D)
+                norms = tuple(copy_to_tp_region(w, self.tp_group) for w in norms)
+        heads = ops.qkv_heads(qkv, batch.position_ids, rope[0], rope[1], Hq, Hk, D, norms, cfg.rms_norm_eps)
+        if heads is None:
+            if norms is not None:
+                q, k, v = qkv.split([cfg.q_size, cfg.kv_size, cfg.kv_size], dim=-1)
+                q, _ = ops.rmsnorm(q.reshape(T * Hq, D), norms[0], cfg.rms_norm_eps)
+                k, _ = ops.rmsnorm(k.reshape(T * Hk, D), norms[1], cfg.rms_norm_eps)
+                qkv = torch.cat([q.reshape(T, -1), k.reshape(T, -1), v], dim=-1)
+            qkv = ops.rope_qkv(qkv, batch.position_ids, rope[0], rope[1], Hq, Hk, D, mrope_section=cfg.mrope_section,
+                               mrope_interleaved=cfg.mrope_interleaved)
+            heads = (qkv[:, : cfg.q_size].view(T, Hq, D), qkv[:, cfg.q_size : cfg.q_size + cfg.kv_size].view(T, Hk, D),
+                     qkv[:, cfg.q_size + cfg.kv_size :].view(T, Hk, D))
+        q, k, v = heads
         o = self._attend(q, k, v, batch)
         out = self.o_proj(o.reshape(T, cfg.q_size))
         if self.tp_group is not None:

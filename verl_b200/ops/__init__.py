@@ -4,7 +4,7 @@ reference paths that exist for the CPU test tier."""
 
 from . import _lib
 from .attention import (attention_varlen, decode_workspace, head_norm_rope_, head_norm_rope_kv_write, kv_cache_write, paged_attention,
-                        paged_decode_attention, qk_norm_kv_write)
+                        paged_decode_attention, qk_norm_kv_write, qkv_heads)
 from .delta import delta_rule
 from .gemm import gemm, linear
 from .gla import gated_linear_attention
@@ -23,7 +23,7 @@ __all__ = [
     "attention_varlen", "paged_decode_attention", "kv_cache_write", "decode_workspace", "ppo_loss_fused", "gae",
     "grpo_advantage", "sample", "decode_advance", "adamw_step", "sumsq_into", "clip_coef", "PPO_METRIC_NAMES",
     "paged_attention", "qk_norm_kv_write", "delta_rule", "add_rmsnorm", "clamped_glu", "embedding_scaled",
-    "rmsnorm_add", "gelu_tanh_glu", "head_norm_rope_", "head_norm_rope_kv_write", "latent_attention", "latent_gather", "latent_prefill",
+    "rmsnorm_add", "gelu_tanh_glu", "head_norm_rope_", "qkv_heads", "head_norm_rope_kv_write", "latent_attention", "latent_gather", "latent_prefill",
     "latent_prefill_supported", "latent_queries", "latent_rope_write", "latent_values", "latent_width", "rotate_tails",
     "embedding_normed", "silu_glu", "gelu_rows", "softcap_", "rglru", "RoutedSum", "moe_route", "moe_experts", "moe_combine",
     "activation", "gated_linear_attention", "moe_norm_add",

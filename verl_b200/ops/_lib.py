@@ -40,7 +40,9 @@ _SIGS = {
     "vb_colsum_bf16": ([P, L, I, I, P, P, P], I),
     "vb_rmsnorm_bwd_parts": ([L], I),
     "vb_rmsnorm_bwd": ([P, P, P, P, P, P, P, P, I, L, I, P], I),
-    "vb_head_norm_rope": ([P, L, P, P, P, P, P, F, L, I, I, I, P, P, P, I, P], I),
+    "vb_head_norm_rope": ([P, L, P, L, P, P, P, P, P, F, L, I, I, I, P, P, P, I, P], I),
+    "vb_head_norm_rope_bwd_parts": ([], I),
+    "vb_head_norm_rope_bwd": ([P, P, P, P, L, P, P, P, P, P, F, L, I, I, I, P, P, P, P, I, I, P], I),
     "vb_rope": ([P, P, L, L, P, P, P, I, I, I, I, I, P], I),
     "vb_mrope": ([P, P, L, L, P, P, P, I, I, I, I, I, I, I, P], I),
     "vb_swiglu_fwd": ([P, P, L, I, P, P], I),

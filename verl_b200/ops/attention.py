@@ -243,26 +243,84 @@ def rotate_pairs(x: torch.Tensor, positions: torch.Tensor, freqs: torch.Tensor, 
     return torch.cat((r, x[..., 2 * n :]), -1)
 
 
+def _head_norm_rope_ok(qkv, pos, cos_t, sin_t, D, norms) -> bool:
+    return (qkv.is_cuda and qkv.dtype == torch.bfloat16 and D in (64, 128, 256) and pos.dim() == 1 and pos.dtype == torch.long
+            and qkv.dim() == 2 and qkv.stride(1) == 1 and qkv.stride(0) % 4 == 0 and qkv.data_ptr() % 8 == 0
+            and cos_t.shape[1] == D // 2 and cos_t.is_contiguous() and sin_t.is_contiguous()
+            and all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.data_ptr() % 8 == 0 for w in norms or ()))
+
+
+def _head_norm_rope(qkv, out, pos, cos_t, sin_t, Hq, Hk, D, norms, eps, slots=None, k_cache=None, v_cache=None):
+    qw, kw = norms or (None, None)
+    rc = _lib.fn("vb_head_norm_rope")(qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), pos.data_ptr(), cos_t.data_ptr(),
+                                      sin_t.data_ptr(), _lib.ptr(qw), _lib.ptr(kw), float(eps), qkv.shape[0], Hq, Hk, D, _lib.ptr(slots),
+                                      _lib.ptr(k_cache), _lib.ptr(v_cache), 0 if k_cache is None else k_cache.shape[2], _lib.stream())
+    _lib.check(rc, "vb_head_norm_rope")
+
+
 def head_norm_rope_(qkv: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t: torch.Tensor, Hq: int, Hk: int, D: int,
                     norms: tuple | None, eps: float, slots: torch.Tensor | None = None, k_cache: torch.Tensor | None = None,
                     v_cache: torch.Tensor | None = None) -> bool:
     """Serving, in place on packed ``qkv`` [T, (Hq + 2 Hk) * D]: RMS norm of every q and k head (``norms`` = weights [D] of q and of
-    k), rotate-half positions, and with ``slots`` the keys and values to the paged caches [NB, Hk, BS, D]; one kernel, one rounding.
+    k), rotate-half positions, and with ``slots`` the keys and values to the paged caches [NB, Hk, BS, D]; one kernel.
     False where it does not apply (nothing is done then): host tensors, gradients, other sizes, multimodal positions."""
-    if (not qkv.is_cuda or torch.is_grad_enabled() or qkv.dtype != torch.bfloat16 or D not in (64, 128, 256) or pos.dim() != 1
-            or pos.dtype != torch.long or qkv.dim() != 2 or qkv.stride(1) != 1 or qkv.stride(0) % 4 or qkv.data_ptr() % 8
-            or cos_t.shape[1] != D // 2 or not cos_t.is_contiguous() or not sin_t.is_contiguous()
-            or any(w.dtype != torch.bfloat16 or not w.is_contiguous() for w in norms or ())):
+    if torch.is_grad_enabled() or not _head_norm_rope_ok(qkv, pos, cos_t, sin_t, D, norms):
         return False
     if slots is not None and not (k_cache.dtype == v_cache.dtype == torch.bfloat16 and k_cache.is_contiguous() and v_cache.is_contiguous()
                                   and (k_cache.data_ptr() | v_cache.data_ptr()) % 8 == 0):
         return False
-    pos, (qw, kw) = pos.contiguous(), norms or (None, None)
-    rc = _lib.fn("vb_head_norm_rope")(qkv.data_ptr(), qkv.stride(0), pos.data_ptr(), cos_t.data_ptr(), sin_t.data_ptr(), _lib.ptr(qw),
-                                      _lib.ptr(kw), float(eps), qkv.shape[0], Hq, Hk, D, _lib.ptr(slots), _lib.ptr(k_cache),
-                                      _lib.ptr(v_cache), 0 if k_cache is None else k_cache.shape[2], _lib.stream())
-    _lib.check(rc, "vb_head_norm_rope")
+    _head_norm_rope(qkv, qkv, pos.contiguous(), cos_t, sin_t, Hq, Hk, D, norms, eps, slots, k_cache, v_cache)
     return True
+
+
+class _QkvFn(torch.autograd.Function):
+    """(q [T, Hq, D], k, v [T, Hk, D]) of a packed projection after head norms and positions. Norm weights with ``main_grad`` (fp32)
+    get their gradients there."""
+
+    @staticmethod
+    def forward(ctx, qkv, qw, kw, pos, cos_t, sin_t, Hq, Hk, D, eps):
+        T, nq, nk = qkv.shape[0], Hq * D, Hk * D
+        out = torch.empty((T, nq + 2 * nk), dtype=qkv.dtype, device=qkv.device)
+        _head_norm_rope(qkv, out, pos, cos_t, sin_t, Hq, Hk, D, None if qw is None else (qw, kw), eps)
+        ctx.save_for_backward(pos, cos_t, sin_t, *(() if qw is None else (qkv, qw, kw)))
+        ctx.dims = (Hq, Hk, D, eps)
+        return out[:, :nq].view(T, Hq, D), out[:, nq : nq + nk].view(T, Hk, D), out[:, nq + nk :].view(T, Hk, D)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        pos, cos_t, sin_t, *normed = ctx.saved_tensors
+        qkv, qw, kw = normed or (None, None, None)
+        Hq, Hk, D, eps = ctx.dims
+        dq, dk, dv = (g if g.data_ptr() % 8 == 0 else g.clone() for g in (g.contiguous() for g in grads))
+        T, dev = dq.shape[0], dq.device
+        dqkv = torch.empty((T, (Hq + 2 * Hk) * D), dtype=dq.dtype, device=dev)
+        part, sums, main = None, [None, None], [None, None]
+        if qw is not None:
+            part = torch.empty((2, _lib.fn("vb_head_norm_rope_bwd_parts")(), D), dtype=torch.float32, device=dev)
+            main = [getattr(w, "main_grad", None) for w in (qw, kw)]
+            sums = [m if m is not None else torch.zeros(D, dtype=torch.float32, device=dev) for m in main]
+        rc = _lib.fn("vb_head_norm_rope_bwd")(dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), _lib.ptr(qkv), 0 if qkv is None else qkv.stride(0),
+                                              pos.data_ptr(), cos_t.data_ptr(), sin_t.data_ptr(), _lib.ptr(qw), _lib.ptr(kw), float(eps),
+                                              T, Hq, Hk, D, dqkv.data_ptr(), _lib.ptr(part), _lib.ptr(sums[0]), _lib.ptr(sums[1]),
+                                              int(main[0] is not None), int(main[1] is not None), _lib.stream())
+        _lib.check(rc, "vb_head_norm_rope_bwd")
+        dws = [None if qw is None or m is not None else s.to(qw.dtype) for s, m in zip(sums, main)]
+        return dqkv, *dws, None, None, None, None, None, None, None
+
+
+def qkv_heads(qkv: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t: torch.Tensor, Hq: int, Hk: int, D: int,
+              norms: tuple | None, eps: float):
+    """q [T, Hq, D], k and v [T, Hk, D] of a packed projection ``qkv`` [T, (Hq + 2 Hk) * D] that nothing else reads, after head norms
+    (``norms``: weights of q and of k, or None) and rotate-half positions; forward and backward are one pass each. None where that does
+    not apply: host tensors, other sizes or types, multimodal positions."""
+    if not _head_norm_rope_ok(qkv, pos, cos_t, sin_t, D, norms):
+        return None
+    pos, (qw, kw) = pos.contiguous(), norms or (None, None)
+    if not _lib.plain():
+        return _QkvFn.apply(qkv, qw, kw, pos, cos_t, sin_t, Hq, Hk, D, eps)
+    _head_norm_rope(qkv, qkv, pos, cos_t, sin_t, Hq, Hk, D, norms, eps)
+    T, nq, nk = qkv.shape[0], Hq * D, Hk * D
+    return qkv[:, :nq].view(T, Hq, D), qkv[:, nq : nq + nk].view(T, Hk, D), qkv[:, nq + nk :].view(T, Hk, D)
 
 
 def head_norm_rope_kv_write(qkv: torch.Tensor, q_weight: torch.Tensor | None, k_weight: torch.Tensor | None,
