@@ -621,11 +621,17 @@ class NativeEngine(BaseEngine):
         if self.device.type != "cuda":
             return 0
         c = self.model_config
-        if c.num_experts:  # routed activations depend on the routing: recompute
-            return 0
+        if c.num_experts and (self.ep_size > 1 or self.tp_size > 1 or c.hidden_size % 64 or c.moe_intermediate_size % 64):
+            return 0  # what a rank holds depends on the routing, or the layer runs in many pieces: recompute
         qkv = (c.num_attention_heads + 2 * c.num_key_value_heads) * c.head_dim
-        per_token = 2 * (5 * c.hidden_size + qkv + c.num_attention_heads * c.head_dim + 3 * c.intermediate_size) + 64
-        per_layer = int(tokens * per_token * 1.1)
+        per_token = 2 * (5 * c.hidden_size + qkv + c.num_attention_heads * c.head_dim) + 64
+        if c.num_experts:  # rows of the buffer sorted by expert, with the most that padding can add, gate logits, heads before their norm
+            pairs = tokens * c.num_experts_per_tok
+            rows = pairs + min(c.num_experts, pairs) * 127
+            inner = rows * 2 * (2 * c.hidden_size + 3 * c.moe_intermediate_size) + tokens * 2 * (c.num_experts + qkv) + pairs * 32
+        else:
+            inner = tokens * 6 * c.intermediate_size
+        per_layer = int((tokens * per_token + inner) * 1.1)
         if n_layers * per_layer <= 1 << 28:  # 256 MB: kept without asking what is free, which takes 1.6 ms of a small micro-batch's 10
             self.last_kept_layers = n_layers
             return n_layers
