@@ -76,6 +76,30 @@ def test_colsum(T, N):
     assert ((colsum(x).double() - ref).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 600, 2305])
+@pytest.mark.parametrize("I,K", [(8, 8), (24, 72), (4864, 896), (2632, 584), (18944, 264)])
+def test_linear_swiglu(M, I, K):
+    """Few rows, CTA pairs (ragged rows, columns and K) and sizes of neither: the bits of a product and an activation of its own."""
+    from verl_b200 import ops
+
+    torch.manual_seed(M + I)
+    x = torch.randn(M, K + 8, device="cuda").bfloat16()[:, :K]
+    w = (torch.randn(2 * I, K, device="cuda") * 2 * K ** -0.5).bfloat16()
+    with torch.no_grad():
+        got = ops.linear_swiglu(x, w)
+        if M > 16:
+            assert torch.equal(got, ops.swiglu(ops.gemm(x, w)))
+        gate, up = (x.double() @ w.double().t()).chunk(2, -1)
+        ref = torch.nn.functional.silu(gate) * up
+        # gate and up rounded (2^-8 each, silu's slope is below 1.1) after fp32 sums of K products, the result rounded
+        silu, sums = torch.nn.functional.silu(gate).abs(), (x.double().abs() @ w.double().abs().t()) * K * 2.0 ** -24
+        e_gate, e_up = (2.0 ** -8 * t.abs() + e for t, e in zip((gate, up), sums.chunk(2, -1)))
+        bound = 1.05 * (1.1 * e_gate * up.abs() + silu * e_up + 1.1 * e_gate * e_up + 2.0 ** -8 * ref.abs()) + 1e-30
+        assert ((got.double() - ref).abs() <= bound).all()
+    leaf = w.clone().requires_grad_(True)
+    assert ops.linear_swiglu(x, leaf).requires_grad
+
+
 def test_gemm_fp32_accumulate_and_bias():
     from verl_b200.ops import gemm
 

@@ -25,28 +25,32 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 constexpr int SK_WARPS = 8;
 
 // NT: groups of 8 rows of A; RT: groups of 16 rows of B per warp; UB: 64-wide steps of k whose loads are in flight together.
-template <int NT, int RT, int UB>
+// GLU (RT 2): B = [gate; up], 2 N rows; a block takes the same 16 rows of both and stores silu(gate) * up of their sums, rounded to bf16
+// first as a product of its own would store them.
+template <int NT, int RT, int UB, bool GLU = false>
 __global__ void __launch_bounds__(SK_WARPS * 32, 2)
 gemm_skinny_kernel(const __nv_bfloat16* A, const __nv_bfloat16* B, void* __restrict__ C, const __nv_bfloat16* bias, int M, int N, int K,
                    long long lda, long long ldb, long long ldc, int out_fp32) {
   constexpr int ROWS = 16 * RT, COLS = 8 * NT;
   __shared__ float red[SK_WARPS][ROWS][COLS + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * ROWS;
+  const int n0 = blockIdx.x * (GLU ? 16 : ROWS);
+  static_assert(!GLU || RT == 2, "16 rows of gate and of up");
+  // row `i` of the block in B; rows past the ends repeat the last one: their sums are not stored
+  auto row_of = [&](int i) { return GLU ? min(n0 + (i & 15), N - 1) + (i >> 4) * N : min(n0 + i, N - 1); };
   pdl_trigger();
   {
     const int lines = (K + 63) >> 6;  // of 128 bytes per row
     for (int i = threadIdx.x; i < ROWS * lines && i < 4 * SK_WARPS * 32; i += SK_WARPS * 32) {
-      const __nv_bfloat16* p = B + (long long)min(n0 + i % ROWS, N - 1) * ldb + (i / ROWS) * 64;
+      const __nv_bfloat16* p = B + (long long)row_of(i % ROWS) * ldb + (i / ROWS) * 64;
       asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
     }
   }
   pdl_wait();
-  // rows past the ends repeat the last one: their sums are not stored
   const __nv_bfloat16* b[RT * 2];
   const __nv_bfloat16* a[NT];
 #pragma unroll
-  for (int r = 0; r < RT * 2; ++r) b[r] = B + (long long)min(n0 + r * 8 + g, N - 1) * ldb + t * 8;
+  for (int r = 0; r < RT * 2; ++r) b[r] = B + (long long)row_of(r * 8 + g) * ldb + t * 8;
 #pragma unroll
   for (int j = 0; j < NT; ++j) a[j] = A + (long long)min(j * 8 + g, M - 1) * lda + t * 8;
   float acc[RT][NT][4] = {};
@@ -84,6 +88,22 @@ gemm_skinny_kernel(const __nv_bfloat16* A, const __nv_bfloat16* B, void* __restr
 #pragma unroll
       for (int i = 0; i < 4; ++i) red[warp][r * 16 + (i >> 1) * 8 + g][j * 8 + 2 * t + (i & 1)] = acc[r][j][i];
   __syncthreads();
+  if (GLU) {
+    for (int i = threadIdx.x; i < 16 * COLS; i += SK_WARPS * 32) {
+      const int n = n0 + i % 16, m = i / 16;
+      if (n >= N || m >= M) continue;
+      float gt = 0.f, up = 0.f;
+#pragma unroll
+      for (int v = 0; v < SK_WARPS; ++v) {
+        gt += red[v][i % 16][m];
+        up += red[v][ROWS - 16 + i % 16][m];
+      }
+      gt = __bfloat162float(__float2bfloat16(gt));
+      up = __bfloat162float(__float2bfloat16(up));
+      reinterpret_cast<__nv_bfloat16*>(C)[m * ldc + n] = __float2bfloat16(gt / (1.f + __expf(-gt)) * up);
+    }
+    return;
+  }
   for (int i = threadIdx.x; i < ROWS * COLS; i += SK_WARPS * 32) {
     const int n = n0 + i % ROWS, m = i / ROWS;
     if (n >= N || m >= M) continue;
@@ -133,6 +153,20 @@ extern "C" int vb_gemm_skinny(const void* A, const void* B, void* C, const void*
   else if (M <= 24) VB_SKINNY(3, 1, 1);
   else if (two) VB_SKINNY(4, 2, 1);
   else VB_SKINNY(4, 1, 1);
+#undef VB_SKINNY
+  vb_count_launch();
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+// C [M, I] = silu(A . W[:I]^T) * (A . W[I:]^T) for up to 16 rows, rows and pointers as vb_gemm_skinny takes them.
+int vb_gemm_skinny_swiglu(const void* A, const void* W, void* C, int M, int I, int K, long long lda, long long ldw, long long ldc,
+                          cudaStream_t stream) {
+  cudaError_t e;
+#define VB_SKINNY(NT, UB)                                                                                                        \
+  e = vb_launch_pdl(gemm_skinny_kernel<NT, 2, UB, true>, dim3((I + 15) / 16), dim3(SK_WARPS * 32), 0, stream, 1,                    \
+                    (const __nv_bfloat16*)A, (const __nv_bfloat16*)W, C, (const __nv_bfloat16*)nullptr, M, I, K, lda, ldw, ldc, 0)
+  if (M <= 8) VB_SKINNY(1, 2);
+  else VB_SKINNY(2, 2);
 #undef VB_SKINNY
   vb_count_launch();
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();

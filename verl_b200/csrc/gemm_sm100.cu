@@ -829,7 +829,10 @@ constexpr int P_STAGE_BYTES = P_A_BYTES + P_B_BYTES;
 constexpr int P_BAR_OFFSET = P_STAGES * P_STAGE_BYTES;
 constexpr int P_DYN_BYTES = P_BAR_OFFSET + (2 * P_STAGES + 4) * 8 + 16 + 1024;
 
-template <bool A_MN, bool B_MN>
+// GLU: B = [gate; up], 2 N rows, and C = silu(A . gate^T) * (A . up^T), both factors rounded to bf16 first as a product of its own would
+// store them. CTA 0 stages 128 rows of gate and CTA 1 the same rows of up, so a tile's accumulator holds both factors of 128 columns:
+// the gate | up activations never reach memory (3584 -> 2 x 18944 on 16 000 tokens: 1.2 GB written and read again by a kernel of 290 us).
+template <bool A_MN, bool B_MN, bool GLU = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -847,7 +850,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 issues the MMAs
   const int num_m2 = (p.M + 2 * BM - 1) / (2 * BM);
-  const int num_n = (p.N + P_BN - 1) / P_BN;
+  constexpr int TILE_N = GLU ? P_BN / 2 : P_BN;  // columns of C per tile
+  const int num_n = (p.N + TILE_N - 1) / TILE_N;
   const int num_units = num_m2 * num_n;
   const int num_kb = (p.K + BK - 1) / BK;
   const int first_unit = (int)cluster_id_x();
@@ -901,7 +905,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         int m2, nb;
         unit_coords(u, m2, nb);
         const int m0 = (2 * m2 + (int)rank) * BM;
-        const int n0 = nb * P_BN + (int)rank * (P_BN / 2);
+        const int n0 = GLU ? nb * TILE_N + (int)rank * p.N : nb * P_BN + (int)rank * (P_BN / 2);
         for (int kb = 0; kb < num_kb; ++kb) {
           if (*abort_flag || !mbar_wait(&empty[s], phase ^ 1)) {
             report_error(p.status, ERR_WAIT_EMPTY, kb);
@@ -1008,11 +1012,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * P_BN;
 #pragma unroll 1
-      for (int c = 0; c < P_BN / 32; ++c) {
+      for (int c = 0; c < TILE_N / 32; ++c) {
         uint32_t r[32];
         tmem_ld_32x32(t_row + c * 32, r);
-        tmem_ld_wait();
-        const int col0 = nb * P_BN + c * 32;
+        if (GLU) {
+          uint32_t up[32];
+          tmem_ld_32x32(t_row + TILE_N + c * 32, up);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const float gt = __bfloat162float(__float2bfloat16(__uint_as_float(r[i])));
+            r[i] = __float_as_uint(gt / (1.f + __expf(-gt)) * __bfloat162float(__float2bfloat16(__uint_as_float(up[i]))));
+          }
+        } else {
+          tmem_ld_wait();
+        }
+        const int col0 = nb * TILE_N + c * 32;
         if (row_ok && col0 < p.N) epi_store_chunk(p, row, col0, r);
       }
       tc_fence_before();
@@ -1034,7 +1049,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool GLU = false>
 static int launch_gemm_pair(const void* A, const void* B, long long lda, long long ldb, const GemmParams& p,
                             cudaStream_t stream) {
   CUtensorMap tmA, tmB;
@@ -1043,9 +1058,9 @@ static int launch_gemm_pair(const void* A, const void* B, long long lda, long lo
   else rc = vb_make_tmap_2d(&tmA, A, 2, (uint64_t)p.K, (uint64_t)p.M, (uint64_t)lda * 2, BK, BM);
   if (rc) return rc;
   if (B_MN) rc = vb_make_tmap_2d(&tmB, B, 2, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)ldb * 2, 64, BK);
-  else rc = vb_make_tmap_2d(&tmB, B, 2, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)ldb * 2, BK, P_BN / 2);
+  else rc = vb_make_tmap_2d(&tmB, B, 2, (uint64_t)p.K, (uint64_t)p.N * (GLU ? 2 : 1), (uint64_t)ldb * 2, BK, P_BN / 2);
   if (rc) return rc;
-  auto kern = gemm_pair_kernel<A_MN, B_MN>;
+  auto kern = gemm_pair_kernel<A_MN, B_MN, GLU>;
   static int max_clusters = 0;  // clusters of two that the device can hold at once (per instantiation)
   if (max_clusters == 0) {
     VB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, P_DYN_BYTES));
@@ -1068,7 +1083,7 @@ static int launch_gemm_pair(const void* A, const void* B, long long lda, long lo
     max_clusters = n;
   }
   if (max_clusters < 0) return -7;
-  const int units = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + P_BN - 1) / P_BN);
+  const int units = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + (GLU ? P_BN / 2 : P_BN) - 1) / (GLU ? P_BN / 2 : P_BN));
   if (units <= 0) return 0;
   const int clusters = units < max_clusters ? units : max_clusters;
   cudaError_t e = vb_launch_pdl(kern, dim3(2 * clusters), dim3(NUM_THREADS), P_DYN_BYTES, stream, 1, tmA, tmB, p);
@@ -1195,6 +1210,14 @@ extern "C" int vb_gemm_skinny(const void* A, const void* B, void* C, const void*
 // ws / counters (optional): fp32 workspace of ws_bytes and num_counters zeroed ints that enable split-K for
 // problems with too few output tiles to occupy the GPU (decode-time projections: M <= 128, large K). Calls
 // that share a workspace must be ordered on one stream. The counters are left at zero.
+static bool pair_enabled() {
+  static const bool on = []() {
+    const char* e = getenv("VERL_B200_GEMM_PAIR");
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
+
 static int gemm_bf16_run(const void* A, const void* B, void* C, const void* bias, int M, int N, int K,
                          long long lda, long long ldb, long long ldc, int a_mn, int b_mn, int out_fp32,
                          int accumulate, float* ws, long long ws_bytes, int* counters, int num_counters,
@@ -1309,11 +1332,7 @@ static int gemm_bf16_run(const void* A, const void* B, void* C, const void* bias
     }
   }
   // Large problems: CTA pairs on 256 x 256 tiles (enough tiles to keep every pair busy for several rounds).
-  static const bool pair_enabled = []() {
-    const char* e = getenv("VERL_B200_GEMM_PAIR");
-    return !(e && e[0] == '0');
-  }();
-  if (pair_enabled && !p.rs_stage && M >= 512 && N >= 512 && K >= 256 &&
+  if (pair_enabled() && !p.rs_stage && M >= 512 && N >= 512 && K >= 256 &&
       (long long)((M + 255) / 256) * ((N + 255) / 256) >= vb_num_sms()) {
     int rc;
     if (!a_mn && !b_mn) rc = launch_gemm_pair<false, false>(A, B, lda, ldb, p, stream);
@@ -1355,6 +1374,30 @@ extern "C" int vb_gemm_bf16_ws(const void* A, const void* B, void* C, const void
                                int* status, cudaStream_t stream) {
   return gemm_bf16_run(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, ws, ws_bytes, counters,
                        num_counters, status, stream, nullptr, 0, 0);
+}
+
+// Gated product C [M, I] = silu(A . W[:I]^T) * (A . W[I:]^T), W = [2 I, K] = gate | up, bf16 (both factors rounded to bf16, as swiglu
+// of a product finds them). vb_gemm_swiglu_ok: 1 few rows (gemm_skinny.cu), 2 CTA pairs, 0 neither: a product and an activation.
+// Pairs under the rule of the plain product; up to 16 rows because a decode step's chain is shorter by a launch then.
+int vb_gemm_skinny_swiglu(const void* A, const void* W, void* C, int M, int I, int K, long long lda, long long ldw, long long ldc,
+                          cudaStream_t stream);
+extern "C" int vb_gemm_swiglu_ok(int M, int I, int K) {
+  if (M <= 0 || I <= 0 || K <= 0 || (I & 7) || (K & 7)) return 0;
+  if (M <= 16) return 1;
+  return pair_enabled() && M >= 512 && I >= 256 && K >= 256 &&
+         (long long)((M + 255) / 256) * ((2ll * I + 255) / 256) >= vb_num_sms() ? 2 : 0;
+}
+extern "C" int vb_gemm_swiglu(const void* A, const void* W, void* C, int M, int I, int K, long long lda, long long ldw, long long ldc,
+                              int* status, cudaStream_t stream) {
+  const int how = vb_gemm_swiglu_ok(M, I, K);
+  if (how == 0 || ((lda | ldw | ldc) & 7) || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(C)) & 15))
+    return -3;
+  if (how == 1) return vb_gemm_skinny_swiglu(A, W, C, M, I, K, lda, ldw, ldc, stream);
+  GemmParams p{};
+  p.M = M; p.N = I; p.K = K;
+  p.C = C; p.ldc = ldc; p.status = status;
+  p.k_splits = 1;
+  return launch_gemm_pair<false, false, true>(A, W, lda, ldw, p, stream);
 }
 
 // GEMM -> reduce-scatter, first half: C = A [M, K] . B [N, K]^T is this rank's partial sum of a row-parallel linear

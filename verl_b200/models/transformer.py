@@ -114,6 +114,8 @@ class DenseMLP(nn.Module):
 
             x = copy_to_tp_region(x, self.tp_group)
             return reduce_from_tp_region(self.down_proj(ops.swiglu(self.gate_up_proj(x))), self.tp_group)
+        if "lora_A" not in self.gate_up_proj.__dict__ and self.gate_up_proj.bias is None:
+            return self.down_proj(ops.linear_swiglu(x, self.gate_up_proj.weight))
         return self.down_proj(ops.swiglu(self.gate_up_proj(x)))
 
     def forward(self, x):

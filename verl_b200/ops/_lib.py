@@ -31,6 +31,8 @@ _SIGS = {
     # gemm
     "vb_gemm_bf16": ([P, P, P, P, I, I, I, L, L, L, I, I, I, I, P, P], I),
     "vb_gemm_bf16_ws": ([P, P, P, P, I, I, I, L, L, L, I, I, I, I, P, L, P, I, P, P], I),
+    "vb_gemm_swiglu_ok": ([I, I, I], I),
+    "vb_gemm_swiglu": ([P, P, P, I, I, I, L, L, L, P, P], I),
     "vb_lmhead_num_splits": ([I, I], I),
     "vb_lmhead_logprob_fwd": ([P, P, P, I, I, I, F, P, P, P, P, P, P, P], I),
     "vb_lmhead_dlogits": ([P, P, P, I, I, I, I, F, P, P, P, P, P, L, P, P], I),

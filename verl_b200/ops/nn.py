@@ -249,6 +249,23 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     return F.silu(g) * u
 
 
+def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """``swiglu(linear(x, weight))`` of a gate | up matrix [2 I, K], in one kernel where nothing records the product: the same bits."""
+    if _lib.plain() and x.is_cuda and x.dim() == 2 and x.dtype == weight.dtype == torch.bfloat16 and weight.shape[0] % 2 == 0:
+        (M, K), I = x.shape, weight.shape[0] // 2
+        if (K == weight.shape[1] and _lib.fn("vb_gemm_swiglu_ok")(M, I, K) and x.stride(1) == weight.stride(1) == 1
+                and (x.stride(0) | weight.stride(0)) % 8 == 0 and (x.data_ptr() | weight.data_ptr()) % 16 == 0):
+            out = torch.empty((M, I), dtype=x.dtype, device=x.device)
+            rc = _lib.fn("vb_gemm_swiglu")(x.data_ptr(), weight.data_ptr(), out.data_ptr(), M, I, K, x.stride(0), weight.stride(0), I,
+                                           _lib.status_word(x.device).data_ptr(), _lib.stream())
+            if rc != -7:  # -7: the device cannot hold the CTA pairs
+                _lib.check(rc, "vb_gemm_swiglu")
+                return out
+    from .gemm import linear
+
+    return swiglu(linear(x, weight))
+
+
 # ------------------------------------------------------------------------- Embedding
 class _EmbeddingFn(torch.autograd.Function):
     @staticmethod

@@ -611,8 +611,9 @@ class NativeRolloutEngine:
             if c.is_moe or not c.mlp_gated:  # routed experts / the two-matrix xIELU MLP: the module's own forward
                 d = self._to_partial(layer.mlp(x), 1, path)
             else:
-                d = self._mm_partial(ops.swiglu(self._mm(x, layer.mlp.gate_up_proj.weight)), layer.mlp.down_proj.weight,
-                                     1, path)
+                w = layer.mlp.gate_up_proj.weight
+                act = ops.linear_swiglu(x, w) if self.on_gpu and id(w) not in self._fp8 else ops.swiglu(self._mm(x, w))
+                d = self._mm_partial(act, layer.mlp.down_proj.weight, 1, path)
             if inject and li in inject and (self.tp == 1 or self.tp_rank == 0):
                 # ``d`` is this rank's partial sum under tensor parallelism: one rank adds the (replicated) values
                 d.index_add_(0, inject[li][0], inject[li][1].to(d.dtype))
