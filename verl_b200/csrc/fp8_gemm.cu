@@ -277,7 +277,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // ------------------------------------------------------------------------------------------------ decode
 // C^T tile [128 rows of W, NT rows of X] per cluster of `splits` CTAs, each with its part of the k blocks. What bounds it is reading W
 // once; the kernel above read 68 MB on 28 SMs with a promotion of 128 columns per k block (48 rows of X; 18 944 -> 3584: 69 us, now
-// 25, floor 11). Partial products wait in F8S_BUFS tensor-memory buffers; the fp32 sums of a cluster meet in shared memory, in slice
+// 18, floor 11). Partial products wait in F8S_BUFS tensor-memory buffers; the fp32 sums of a cluster meet in shared memory, in slice
 // order. The first rows of W are asked for in L2 while the kernel before still runs (a hint, it may come before the wait).
 constexpr int F8S_BUFS = 4;
 template <int NT>
@@ -509,34 +509,6 @@ fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_con
   }
 }
 
-// How many clusters of `cluster` CTAs of the kernel the device holds at once (asked once per size and device).
-template <int NT>
-static int fp8_skinny_clusters(int cluster) {
-  static int cache[64][9];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (cache[dev][cluster] == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cluster * 64);
-    cfg.blockDim = dim3(F8_THREADS);
-    cfg.dynamicSmemBytes = F8Skinny<NT>::SMEM;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = cluster;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, fp8_gemm_skinny_kernel<NT>, &cfg) != cudaSuccess || n <= 0) {
-      (void)cudaGetLastError();
-      n = -1;
-    }
-    cache[dev][cluster] = n;
-  }
-  return cache[dev][cluster];
-}
-
 template <int NT>
 static int launch_fp8_skinny(const void* xq, const void* wq, long long ldx, long long ldw, const F8Params& p, cudaStream_t stream) {
   using L = F8Skinny<NT>;
@@ -553,12 +525,14 @@ static int launch_fp8_skinny(const void* xq, const void* wq, long long ldx, long
     VB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM));
     if (dev >= 0 && dev < 64) attr_set[dev] = true;
   }
-  // the most CTAs of one wave (two per SM), six k blocks or more per CTA: below, the cluster's exchange costs more than it gives
+  // The most CTAs of about one wave (two per SM, less what clusters leave idle in a part of the chip: 288 of 296 took longer than 216),
+  // six k blocks or more per CTA: below, the cluster's exchange costs more than it gives. Waves are not asked from the occupancy
+  // calculator: it allowed 28 clusters of four where 28 of eight run (18 944 -> 3584, 48 rows: 25.5 against 17.8 us).
   const int m_tiles = (p.M + NT - 1) / NT, tiles = (p.N + 127) / 128 * m_tiles, nkb = (p.K + F8_BK - 1) / F8_BK;
   int splits = 1, per = nkb;
-  for (int s = 2; s <= 8 && s * 6 <= nkb && tiles * s <= 2 * vb_num_sms(); ++s) {
+  for (int s = 2; s <= 8 && s * 6 <= nkb && tiles * s * 4 <= 7 * vb_num_sms(); ++s) {
     const int each = (nkb + s - 1) / s;
-    if ((nkb + each - 1) / each != s || tiles > fp8_skinny_clusters<NT>(s)) continue;
+    if ((nkb + each - 1) / each != s) continue;
     splits = s;
     per = each;
   }
@@ -607,8 +581,8 @@ extern "C" int vb_fp8_gemm_blockscale(const void* xq, const void* wq, const floa
   p.C = reinterpret_cast<__nv_bfloat16*>(C); p.ldc = ldc;
   p.sx = sx; p.sw = sw; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias); p.status = status;
   // us, the kernel below -> the decode kernel (M = 1 / 48 / 64 / 96 / 128):
-  //   3584 -> 4608   16 -> 7.7 / 10 / 12 / 12 / 14    18944 -> 3584  68 -> 19 / 25 / 31 / 45 / 57    4096 -> 6144  18 -> 10 / 13 / 16 / 22 / 27
-  //   3584 -> 37888  36 -> 23 / 26 / 28 / 41 / 48     4096 -> 28672  40 -> 21 / 27 / 32 / 49 / 61    4864 -> 896   20 -> 6.1 / 7.6 / 8.3 / 8.2 / 9.5
+  //   3584 -> 4608   16 -> 7.0 / 8.9 / 10 / 12 / 14   18944 -> 3584  68 -> 14 / 18 / 22 / 26 / 33   4096 -> 6144  18 -> 8.1 / 11 / 13 / 19 / 20
+  //   3584 -> 37888  36 -> 24 / 26 / 28 / 34 / 34     4096 -> 28672  40 -> 21 / 27 / 32 / 36 / 37    4864 -> 896   20 -> 6.2 / 7.6 / 8.5 / 8.3 / 9.5
   // More than 64 rows of X are two tiles, which read W twice (from L2): worth it while all tiles together leave half of the SMs
   // without one, so that the kernel below would, too.
   if (M <= 16) return launch_fp8_skinny<16>(xq, wq, ldx, ldw, p, stream);
