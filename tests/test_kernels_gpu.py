@@ -65,6 +65,38 @@ def test_gemm_few_rows(M, N, K):
     assert ((got - want).abs() <= bound + 2.0 ** -8 * want.abs() + 2.0 ** -23).all()
 
 
+@pytest.mark.parametrize("M", [1, 8, 16, 32])
+def test_gemm_few_rows_of_operands_just_written(M):
+    """Both operands of a few-row product come from the kernels right before it, into the same buffers again and again: the bits are
+    those of the ordinary stream order, where no kernel starts before the one before it has ended."""
+    from verl_b200 import ops
+    from verl_b200.ops import _lib
+
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()  # noqa: E731
+    K, N = 1024, 264
+    xs, ys, wa, wb = rnd(12, M, 512), rnd(12, N, 512), rnd(K, 512), rnd(K, 512)
+
+    def passes():
+        a, b = (torch.zeros(r, K, device="cuda", dtype=torch.bfloat16) for r in (M, N))
+        outs = []
+        for x, y in zip(xs, ys):
+            ops.gemm(y, wb, out=b)  # the matrix, by the tile kernel
+            ops.gemm(x, wa, out=a)  # the rows, by the few-row kernel itself
+            outs.append(ops.gemm(a, b, out_dtype=torch.float32))
+            ops.gemm(y[:M], wb, out=b[:M])  # part of the matrix by the kernel right before
+            outs.append(ops.gemm(a, b, out_dtype=torch.float32))
+        return torch.stack(outs)
+
+    try:
+        _lib.set_pdl(False)
+        want = passes()
+    finally:
+        _lib.set_pdl(True)
+    for _ in range(3):
+        assert torch.equal(passes(), want)
+
+
 @pytest.mark.parametrize("T,N", [(1, 2), (7, 34), (8, 512), (511, 514), (512, 1026), (3000, 4608), (5, 33)])
 def test_colsum(T, N):
     from verl_b200.ops.gemm import colsum

@@ -48,3 +48,25 @@ def test_python_calls_only_exported_native_functions():
         used |= set(re.findall(r"""["'.](vb_[a-z0-9_]+)""", py.read_text()))
     missing = sorted(u for u in used if u not in defined)
     assert not missing, missing
+
+
+def test_kernels_that_start_early_use_no_read_only_loads():
+    """A kernel that waits for the one before it (``pdl_wait``) has begun while that one still writes: what it reads of it may not go
+    through loads that promise memory nobody writes. Model weights and position tables, which no such kernel writes, may."""
+    constant = {"w", "qw", "kw", "cos_t", "sin_t", "post"}
+    found, seen = [], 0
+    for name in ("elementwise.cu", "fp8_gemm.cu", "gemm_skinny.cu", "moe_ops.cu", "paged_attention.cu", "paged_attention_mma.cu"):
+        src = (ROOT / "verl_b200" / "csrc" / name).read_text()
+        for kernel in src.split("__global__")[1:]:
+            kernel = kernel.split("\n}\n")[0]
+            head, _, body = kernel.partition("{\n")
+            if "pdl_wait()" not in body:
+                continue
+            seen += 1
+            params = re.findall(r"const [\w:]+\*\s*__restrict__\s+(\w+)", head)
+            found += [(name, head.split("(")[0].split()[-1], p) for p in params if p not in constant]
+            if "ld_stream(" in body:
+                body += src.split("uint4 ld_stream(")[1].split("\n}\n")[0]
+                assert "asm volatile" in body and '"memory"' in body
+            found += [(name, w) for w in ("__ldg(", "ld.global.nc") if w in body]
+    assert seen >= 12 and not found, (seen, found)

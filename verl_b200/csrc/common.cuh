@@ -82,7 +82,10 @@ __device__ __forceinline__ bool elect_one() {
 // its predecessor in the stream still runs: what it does before pdl_wait() (barrier init, TMEM allocation,
 // descriptor prefetch) overlaps the predecessor's tail. pdl_wait() returns once every prerequisite grid has
 // finished and its writes are visible; no global memory that another kernel produces or reads may be touched
-// before it. pdl_trigger() lets the NEXT kernel be scheduled; call it only after this CTA holds every resource it
+// before it. That binds the compiler too: what the kernel before may write is read by plain loads (no __ldg, no
+// ld.global.nc, no `const T* __restrict__`: they promise memory that nobody writes while the kernel lives, and such
+// loads need not stay behind the wait). pdl_trigger() lets the NEXT kernel be scheduled; call it only after this CTA
+// holds every resource it
 // will ever allocate (TMEM above all: a dependent that took the columns first would wait on this kernel while
 // this kernel waits on the columns). Both are no-ops in a kernel launched the ordinary way.
 // ---------------------------------------------------------------------------

@@ -44,7 +44,7 @@ __device__ __forceinline__ float block_reduce_sum(float v, float* sh) {
 
 // ------------------------------- RMSNorm ------------------------------------
 // y = (x [+ res]) * rstd * w ; optionally writes the pre-norm sum to res_out.
-__global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
+__global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* res,
                                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                                    __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out, int H,
                                    float eps) {
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(256) colsum_rows_kernel(const __nv_bfloat16* _
 // (row strides given in elements). cos/sin tables are [max_pos, D/2] fp32.
 // sign = +1 forward, -1 backward (transpose of the rotation).
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ k, long long q_stride,
-                            long long k_stride, const long long* __restrict__ pos, const float* __restrict__ cos_t,
+                            long long k_stride, const long long* pos, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, int T, int Hq, int Hk, int D, float sign, int mrope_s0,
                             int mrope_s1) {
   // multimodal rotary embedding (mrope_s0 > 0): pos is [3, T] (temporal, height, width); rotary frequency j takes the
@@ -392,8 +392,8 @@ __global__ void __launch_bounds__(256) head_norm_rope_bwd_kernel(
 // ------------------------------- SwiGLU --------------------------------------
 // gu: [T, 2I] (gate | up), out: [T, I]
 // blk_expert (null: none): rows of a buffer sorted by expert, blocks of 128 rows without one are left out.
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T,
-                                  int I, const int* __restrict__ blk_expert) {
+__global__ void swiglu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* __restrict__ out, long long T, int I,
+                                  const int* blk_expert) {
   pdl_trigger();
   pdl_wait();
   const int nvec = I >> 3;

@@ -68,7 +68,7 @@ __global__ void fp8_quant_weight_kernel(const __nv_bfloat16* __restrict__ w, lon
 }
 
 // one warp per (row, 128-column block)
-__global__ void fp8_quant_act_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, long long M, int K,
+__global__ void fp8_quant_act_kernel(const __nv_bfloat16* x, long long ldx, long long M, int K,
                                      __nv_fp8_storage_t* __restrict__ q, long long ldq, float* __restrict__ scales, int pow2) {
   pdl_trigger();
   pdl_wait();

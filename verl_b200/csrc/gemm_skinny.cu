@@ -11,9 +11,10 @@
 
 namespace vb {
 
+// Not the read-only path: the kernel before this one may write B (a product of two activations) while this one has begun already.
 __device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {
   uint4 v;
-  asm("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -66,7 +67,7 @@ gemm_skinny_kernel(const __nv_bfloat16* A, const __nv_bfloat16* B, void* __restr
 #pragma unroll
         for (int r = 0; r < RT * 2; ++r) w[u][h][r] = in ? ld_stream(b[r] + k) : zero;
 #pragma unroll
-        for (int j = 0; j < NT; ++j) x[u][h][j] = in ? __ldg(reinterpret_cast<const uint4*>(a[j] + k)) : zero;
+        for (int j = 0; j < NT; ++j) x[u][h][j] = in ? *reinterpret_cast<const uint4*>(a[j] + k) : zero;
       }
 #pragma unroll
     for (int u = 0; u < UB; ++u)

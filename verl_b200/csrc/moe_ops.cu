@@ -171,8 +171,7 @@ __global__ void moe_layout_kernel(const MoeRouteParams p) {
 
 // xs[dest[t, k]] = x[t], scale[dest[t, k]] = weight[t, k]. One block per token.
 template <typename T>
-__global__ void moe_gather_kernel(const T* __restrict__ x, long long stride, const int* __restrict__ dest,
-                                  const float* __restrict__ weight, int top, int H, T* __restrict__ xs,
+__global__ void moe_gather_kernel(const T* x, long long stride, const int* dest, const float* weight, int top, int H, T* __restrict__ xs,
                                   float* __restrict__ scale) {
   __shared__ int to[MR_MAX_TOP];
   pdl_trigger();
@@ -201,9 +200,8 @@ __global__ void moe_gather_kernel(const T* __restrict__ x, long long stride, con
 // y = res / sqrt(mean + eps) * w, or without w the residual. With post: d *= sigmoid(gate[t]) element by element (when given),
 // res += d / sqrt(mean(d^2) + eps) * post, y = res / sqrt(mean + eps) * w * scale. One block per token.
 template <typename T>
-__global__ void moe_combine_kernel(const T* __restrict__ out, const int* __restrict__ dest, const float* __restrict__ weight,
-                                   int top, const T* __restrict__ shared, long long shared_stride,
-                                   const float* __restrict__ logit, long long logit_stride, const T* __restrict__ gate,
+__global__ void moe_combine_kernel(const T* out, const int* dest, const float* weight, int top, const T* shared,
+                                   long long shared_stride, const float* logit, long long logit_stride, const T* gate,
                                    long long gate_stride, const T* __restrict__ post, float* __restrict__ res,
                                    const T* __restrict__ w, float scale, T* __restrict__ y, int H, float eps, bool vec) {
   extern __shared__ float row[];
@@ -271,7 +269,7 @@ __global__ void moe_combine_kernel(const T* __restrict__ out, const int* __restr
 // One warp per token: softmax over the E logits, the k largest (ties: the lowest index, as torch.topk takes them) or the given
 // ones, their probabilities, divided by their sum with `renorm`.
 template <typename T, int NV>
-__global__ void __launch_bounds__(256) moe_gate_kernel(const T* __restrict__ logits, long long stride, int tokens, int E, int k,
+__global__ void __launch_bounds__(256) moe_gate_kernel(const T* logits, long long stride, int tokens, int E, int k,
                                                        int renorm, int given, long long* __restrict__ idx,
                                                        float* __restrict__ weight) {
   pdl_trigger();
@@ -397,7 +395,7 @@ __global__ void __launch_bounds__(256) moe_gate_bwd_kernel(const T* __restrict__
 // block per expert counts all pairs in shared memory (for the offsets) and ranks its own. dest[pair] = row, -1 for pairs of experts
 // outside [first, first + E); src[row] = pair, -1 for the rows that pad an expert's share to a multiple of 128.
 constexpr int MP_MAX_E = 2048, MP_THREADS = 1024;
-__global__ void __launch_bounds__(MP_THREADS) moe_place_kernel(const long long* __restrict__ idx, long long n, int first, int E,
+__global__ void __launch_bounds__(MP_THREADS) moe_place_kernel(const long long* idx, long long n, int first, int E,
                                                                int* __restrict__ dest, int* __restrict__ src,
                                                                int* __restrict__ blk_expert, int nblk, int* __restrict__ expert_off) {
   __shared__ int hist[MP_MAX_E], off[MP_MAX_E + 1], part[2][32];
@@ -454,9 +452,8 @@ __global__ void __launch_bounds__(MP_THREADS) moe_place_kernel(const long long* 
 }
 
 // xs[r] = x[token of the pair src[r]], zeros in padding rows; blocks without an expert are left out. One warp per row.
-__global__ void __launch_bounds__(256) moe_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ src,
-                                                       const int* __restrict__ blk_expert, long long rows, int k, int vecs,
-                                                       uint4* __restrict__ xs) {
+__global__ void __launch_bounds__(256) moe_rows_kernel(const uint4* x, const int* src, const int* blk_expert, long long rows, int k,
+                                                       int vecs, uint4* __restrict__ xs) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -510,8 +507,7 @@ __global__ void __launch_bounds__(256) moe_rows_bwd_kernel(const __nv_bfloat16* 
 
 // y[t] = sum over the slots of w[t, j] * row[dest[t, j]] (w null: of the rows); pairs without a row count nothing. A block takes
 // 8 * blockDim elements of a token.
-__global__ void __launch_bounds__(256) moe_weighted_sum_kernel(const __nv_bfloat16* __restrict__ row, const int* __restrict__ dest,
-                                                               const float* __restrict__ w, int k, int H,
+__global__ void __launch_bounds__(256) moe_weighted_sum_kernel(const __nv_bfloat16* row, const int* dest, const float* w, int k, int H,
                                                                __nv_bfloat16* __restrict__ y) {
   pdl_trigger();
   pdl_wait();

@@ -254,8 +254,7 @@ __global__ void decode_merge_any_kernel(const float* __restrict__ o_part, const 
 }
 
 // k, v: [T, Hk, D] (token stride given); slot = block * block_size + offset, slot < 0 skips the token.
-__global__ void kv_write_kernel(const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
-                                long long k_stride, long long v_stride, const long long* __restrict__ slots,
+__global__ void kv_write_kernel(const __nv_bfloat16* k, const __nv_bfloat16* v, long long k_stride, long long v_stride, const long long* slots,
                                 __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc, long long T, int Hk,
                                 int D, int block_size) {
   pdl_trigger();
