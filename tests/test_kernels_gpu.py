@@ -584,6 +584,31 @@ def test_paged_decode_attention(B, Hq, Hk, D, bs, maxlen):
             _bf16_close(out, ref, ulps=4)
 
 
+@pytest.mark.parametrize("Hq,Hk,D,bs,lens", [(14, 2, 64, 16, (500, 1, 129)), (8, 8, 64, 8, (3000, 17)), (32, 2, 64, 32, (700, 64)),
+                                             (8, 1, 128, 256, (2100, 255, 300)), (9, 1, 128, 512, (513, 30))])
+def test_decode_attention_weights_stay_in_fp32(Hq, Hk, D, bs, lens):
+    """Heads of 64, and pages above 128 rows: the splits' fp32 results against fp64, before anything is rounded to bf16."""
+    from verl_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(Hq + D)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()  # noqa: E731
+    B, G, S = len(lens), Hq // Hk, 3
+    n = (max(lens) + bs - 1) // bs
+    q, kc, vc = rnd(B, Hq, D), rnd(B * n, Hk, bs, D), rnd(B * n, Hk, bs, D)
+    table = torch.arange(B * n, device="cuda", dtype=torch.int32).reshape(B, n)
+    work = torch.zeros(B * Hq * S * (D + 2), device="cuda")
+    ops.paged_decode_attention(q, kc, vc, table, torch.tensor(lens, dtype=torch.int32, device="cuda"), num_splits=S, work=work)
+    o, ml = work[: B * Hq * S * D].view(B, Hq, S, D).double(), work[B * Hq * S * D :].view(B, Hq, S, 2).double()
+    part = torch.exp(ml[..., 0] - ml[..., 0].amax(-1, keepdim=True))
+    got = (o * part[..., None]).sum(2) / (ml[..., 1] * part).sum(-1)[..., None]
+    for b, L in enumerate(lens):
+        k, v = (c.view(B, n, Hk, bs, D)[b].transpose(0, 1).reshape(Hk, n * bs, D)[:, :L].double() for c in (kc, vc))
+        p = torch.softmax(torch.einsum("hgd,hkd->hgk", q[b].view(Hk, G, D).double(), k) * D ** -0.5, -1)
+        want = torch.einsum("hgk,hkd->hgd", p, v).reshape(Hq, D)
+        # scores of up to about 5 in fp32 and sums of L weights: 2^-24 each, some tens of them together; weights in bf16 would be 2^-10 off
+        assert float((got[b] - want).norm() / want.norm()) <= 64 * 2.0 ** -24
+
+
 def _attn_ref(q, k, v, cu, causal, scale):
     """fp32 reference, one sequence at a time. Returns (out [T,Hq,D], lse [Hq,T])."""
     T, Hq, D = q.shape

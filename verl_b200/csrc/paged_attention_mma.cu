@@ -7,12 +7,18 @@
 // (D 64: the CUDA-core kernel), and the time of the bytes:
 //   128 sequences of 430, 28 / 4 heads of 128: 31.8 (47.3; 17.0)     48 of 500: 17.0 (35.1; 7.7)     1 of 8000: 16.4 (19.8; 2.3)
 //   256 of 1000: 99.5 (147.8; 81.5)     128 of 1000, 32 / 8 heads: 95.8 (123.1; 80.5)     16 of 4000: 33.0 (54.0; 20.5)
-//   14 / 2 heads of 64: 1 of 85 2.7 (15.1)     16 of 500 3.7 (21.9; 0.6)     128 of 500 10.4 (89.0; 5.1)
+//   14 / 2 heads of 64: 1 of 85 2.8 (15.8)     16 of 500 5.6 (21.1; 0.6)     128 of 500 9.2 (40.5; 5.1)
 //
 //   S[heads, keys]  = Q[16, D] . K^T   mma.m16n8k16; the order of dims inside a product is free as long as Q and K share it, so a
 //                                      lane's 16 bytes of a key are two steps' operands as they come
-//   O^T[dims, heads] += V^T . P^T      P: the scores' own registers, rounded to bf16; V's operand holds two keys of a dim per
-//                                      register: a lane loads 16 bytes of four keys and pairs them
+//   O^T[dims, heads] += V^T . P^T      P: the scores' own registers, as bf16; V's operand holds two keys of a dim per register: a lane
+//                                      loads 16 bytes of four keys and pairs them
+//
+// Heads of 64, and pages above 128 rows, keep their weights in fp32: three bf16 terms hold all 24 bits, their products of 16 keys are
+// summed on their own and added to the rest with rounding to nearest. Against 64 bits (relative 2-norm before the result is rounded) 1.7e-7
+// to 2.5e-7, on CUDA cores 1.9e-7 to 4.5e-7, with one term 1.2e-3 (which moves a bf16 result from 1.6e-3 to 2.0e-3); one term would be 0.1 to
+// 0.2 us faster. Heads of 128 in smaller pages take one term, as the tcgen05 kernel did (1.2e-3, that one 1.4e-3): three would take 10 to 20 %
+// longer there (128 of 430: 36.8 us, 30.9 with one).
 //
 // Next keys' K loads are in flight while V and the softmax of these are worked on. fp32 softmax, base 2, online per warp.
 #include "common.cuh"
@@ -29,8 +35,8 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
 }
 __device__ __forceinline__ uint32_t word(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
-// HI: more than eight query heads per KV head (rows 8 .. 15 of the products hold some).
-template <int D, bool HI>
+// HI: more than eight query heads per KV head (rows 8 .. 15 of the products hold some). TERMS: bf16 terms that a weight is cut into.
+template <int D, bool HI, int TERMS>
 __global__ void __launch_bounds__(DM_WARPS * 32, HI ? 2 : 3)
 paged_decode_mma_kernel(const __nv_bfloat16* q, long long q_stride, const __nv_bfloat16* kc, const __nv_bfloat16* vc,
                         const int* block_table, int max_blocks, const int* seq_lens, int Hq, int Hk, int shift, float scale_log2,
@@ -135,7 +141,7 @@ paged_decode_mma_kernel(const __nv_bfloat16* q, long long q_stride, const __nv_b
       row[1] = cache_row(key0 + 8);
       load_k();
     }
-    uint32_t p[2][R];  // [eight keys][row]: bf16 pairs
+    uint32_t p[TERMS][2][R];  // [term][eight keys][row]: bf16 pairs
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       float x[4], nm = m[r];
@@ -154,8 +160,14 @@ paged_decode_mma_kernel(const __nv_bfloat16* q, long long q_stride, const __nv_b
         x[i] = exp2f(x[i] - to);
         l[r] += x[i];
       }
-      p[0][r] = pack_bf16x2(x[0], x[1]);
-      p[1][r] = pack_bf16x2(x[2], x[3]);
+#pragma unroll
+      for (int n = 0; n < TERMS; ++n)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          p[n][j][r] = pack_bf16x2(x[2 * j], x[2 * j + 1]);
+          x[2 * j] -= __uint_as_float(p[n][j][r] << 16);
+          x[2 * j + 1] -= __uint_as_float(p[n][j][r] & 0xffff0000u);
+        }
       if (__any_sync(0xffffffffu, alpha != 1.f)) {
         const float a0 = __shfl_sync(0xffffffffu, alpha, 8 * t), a1 = __shfl_sync(0xffffffffu, alpha, 8 * t + 4);  // heads 2t, 2t + 1
 #pragma unroll
@@ -174,7 +186,17 @@ paged_decode_mma_kernel(const __nv_bfloat16* q, long long q_stride, const __nv_b
         const uint32_t a0 = __byte_perm(k0, k1, 0x5410), a1 = __byte_perm(k0, k1, 0x7632);
         const uint32_t a2 = __byte_perm(k2, k3, 0x5410), a3 = __byte_perm(k2, k3, 0x7632);
 #pragma unroll
-        for (int r = 0; r < R; ++r) mma_bf16(acc[r][c][e], a0, a1, a2, a3, p[0][r], p[1][r]);
+        for (int r = 0; r < R; ++r) {
+          if (TERMS == 1) {
+            mma_bf16(acc[r][c][e], a0, a1, a2, a3, p[0][0][r], p[0][1][r]);
+          } else {  // 16 keys on their own, then a sum that is rounded to nearest
+            float part[4] = {};
+#pragma unroll
+            for (int n = TERMS - 1; n >= 0; --n) mma_bf16(part, a0, a1, a2, a3, p[n][0][r], p[n][1][r]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[r][c][e][i] += part[i];
+          }
+        }
       }
   }
 
@@ -244,15 +266,17 @@ extern "C" int vb_paged_decode_mma(const void* q, long long q_stride, const void
   while ((1 << shift) < block_size) ++shift;
   const float scale_log2 = scale * 1.4426950408889634f;
   cudaError_t e;
-#define VB_DM(DD, HI)                                                                                                            \
-  e = vb_launch_pdl(paged_decode_mma_kernel<DD, HI>, dim3(B, Hk, num_splits), dim3(DM_WARPS * 32), 0, stream, 1,                  \
+#define VB_DM(DD, HI, TERMS)                                                                                                     \
+  e = vb_launch_pdl(paged_decode_mma_kernel<DD, HI, TERMS>, dim3(B, Hk, num_splits), dim3(DM_WARPS * 32), 0, stream, 1,           \
                     (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc, block_table, max_blocks, \
                     seq_lens, Hq, Hk, shift, scale_log2, num_splits, (__nv_bfloat16*)out, out_stride, work, ml_part)
   const bool hi = Hq / Hk > 8;
-  if (D == 128 && hi) VB_DM(128, true);
-  else if (D == 128) VB_DM(128, false);
-  else if (hi) VB_DM(64, true);
-  else VB_DM(64, false);
+  if (D == 64 && hi) VB_DM(64, true, 3);
+  else if (D == 64) VB_DM(64, false, 3);
+  else if (block_size > 128 && hi) VB_DM(128, true, 3);
+  else if (block_size > 128) VB_DM(128, false, 3);
+  else if (hi) VB_DM(128, true, 1);
+  else VB_DM(128, false, 1);
 #undef VB_DM
   vb_count_launch(num_splits > 1 ? 2 : 1);
   if (e == cudaSuccess) e = cudaGetLastError();
