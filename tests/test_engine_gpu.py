@@ -28,6 +28,43 @@ def _batch(cfg, lens, dev):
     return PackedBatch(ids.to(dev), pos.to(dev), cu.to(dev), max(lens)), ids
 
 
+def test_replayed_experts_that_the_model_does_not_have_stop_the_update():
+    """The optimizer step raises and takes no step; the one after it, with a sound record, goes through."""
+    import contextlib
+
+    from verl_b200.ops import _lib
+    from verl_b200.workers.engine.native import NativeEngine
+
+    class C(dict):
+        __getattr__ = dict.get
+
+    cfg = _cfg("moe")
+    eng = NativeEngine(cfg, C(), C(lr=1e-3, clip_grad=1.0, weight_decay=0.0), device="cuda", seed=9).initialize()
+    batch, ids = _batch(cfg, [40, 25], "cuda")
+    rows = torch.arange(30, device="cuda")
+    good = torch.arange(65, device="cuda")[:, None] % 7 + torch.arange(2, device="cuda")
+
+    def step(routing):
+        for layer in eng.model.layers:
+            layer.mlp.replay_routing = routing
+        with eng.train_mode():
+            eng.optimizer_zero_grad()
+            lp, _ = eng.forward_logprob(batch, rows, ids.cuda()[rows + 1], 1.0)
+            (-lp.mean()).backward()
+            return eng.optimizer_step()
+
+    before = eng.zero.master.clone()
+    bad = good.clone()
+    bad[3, 1] = cfg.num_experts
+    with pytest.raises(RuntimeError, match="outside"):
+        step(bad)
+    assert torch.equal(eng.zero.master, before)
+    torch.cuda.synchronize()
+    with contextlib.suppress(RuntimeError):  # kernels of the abandoned pass may have noted the index again
+        _lib.raise_refused()
+    assert bool(torch.isfinite(step(good))) and not torch.equal(eng.zero.master, before)
+
+
 @pytest.mark.parametrize("kind", ["dense", "moe"])
 def test_engine_logprob_and_step_match_cpu_fp32(kind):
     from verl_b200.models.transformer import CausalLM

@@ -831,6 +831,49 @@ def test_moe_gate_matches_softmax_topk(E, k, renorm, given):
     assert float((z.grad.double() - zr.grad).abs().max()) <= 2.0 ** -8 * float(zr.grad.abs().max()) + 1e-9
 
 
+@pytest.mark.parametrize("bad", [-1, 8, 1 << 32])
+@pytest.mark.parametrize("renorm", [True, False])
+def test_experts_outside_the_layer_are_refused(bad, renorm):
+    """A given expert that the layer does not have (also one that is 0 in its low 32 bits): the next look raises, once, and until then
+    nothing that depends on it is a number; other tokens are as without it. A replica's part takes them for another rank's."""
+    from verl_b200 import ops
+    from verl_b200.ops import _lib
+    from verl_b200.ops.moe import moe_gate, moe_mlp
+
+    T, E, k, H, I = 12, 8, 2, 64, 64
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    z, x = rnd(T, E), rnd(T, H).bfloat16()
+    gate_up, down = (rnd(*s).bfloat16() * 0.1 for s in ((E, 2 * I, H), (E, H, I)))
+    good = rnd(T, E).topk(k, -1).indices
+    given = good.clone()
+    given[4, 1] = bad
+    keep = torch.arange(T, device="cuda") != 4
+    want = moe_gate(z, k, renorm, good)[0]
+
+    def looked():
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="pair 9 .* outside"):
+            _lib.raise_refused()
+        _lib.raise_refused()
+
+    got = moe_gate(z, k, renorm, given)[0]
+    looked()
+    assert bool(got[4, 1].isnan()) and torch.equal(got[keep], want[keep])
+    leaf = z.clone().requires_grad_(True)
+    w, _ = moe_gate(leaf, k, renorm, given)
+    looked()
+    w.sum().backward()
+    assert bool(leaf.grad[4].isnan().any()) and not bool(leaf.grad[keep].isnan().any())
+    y = moe_mlp(x, given, want, gate_up, down, ops.swiglu)
+    looked()
+    assert bool(y[4].isnan().all()) and torch.equal(y[keep], moe_mlp(x, good, want, gate_up, down, ops.swiglu)[keep])
+    part = moe_mlp(x, given, want, gate_up[2:6].contiguous(), down[2:6].contiguous(), ops.swiglu, expert_offset=2, num_experts=E)
+    torch.cuda.synchronize()
+    _lib.raise_refused()
+    assert not bool(part.isnan().any())
+
+
 def test_bounded_device_wait_reports_status_and_context_survives():
     """A cross-rank barrier whose peer never arrives: the kernel gives up after its time limit, records the wait in
     the status word and returns; the host reads the code and the context keeps working."""

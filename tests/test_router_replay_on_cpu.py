@@ -201,3 +201,16 @@ def test_grpo_with_r3_replay_end_to_end(tmp_path, monkeypatch, agent):
         assert key in m and math.isfinite(m[key]), key
     # same weights and the same experts in the rollout and in the trainer's log-prob pass
     assert m["training/rollout_probs_diff_mean"] < 1e-3
+
+
+def test_a_refused_index_is_raised_once(monkeypatch):
+    import ctypes
+
+    import pytest
+
+    from verl_b200.ops import _lib
+
+    monkeypatch.setattr(_lib, "_refused", (None, (ctypes.c_int * 4)(1, 9, 3, 8)))
+    with pytest.raises(RuntimeError, match=r"index 9 of pair 3 .* outside \[0, 8\)"):
+        _lib.raise_refused()
+    _lib.raise_refused()

@@ -266,12 +266,24 @@ __global__ void moe_combine_kernel(const T* out, const int* dest, const float* w
 // of 2048 with 128 experts of 768: decode step of 24 sequences 2.06 -> 1.26 ms, two layers forward on 6000 tokens 8.68 -> 6.63 ms.
 // ---------------------------------------------------------------------------------------------------------------------------
 
+// An expert that the layer does not have: `refused` (4 ints of host memory, null: none) says so to the next call or optimizer step that
+// looks, and what depends on the pair is no number until then.
+__device__ __forceinline__ void refuse_expert(int* refused, long long e, long long pair, int E) {
+  if (refused == nullptr) return;
+  volatile int* r = refused;
+  r[1] = (int)min(max(e, -0x7fffffffLL), 0x7fffffffLL);
+  r[2] = (int)min(pair, 0x7fffffffLL);
+  r[3] = E;
+  __threadfence_system();
+  r[0] = 1;
+}
+
 // One warp per token: softmax over the E logits, the k largest (ties: the lowest index, as torch.topk takes them) or the given
-// ones, their probabilities, divided by their sum with `renorm`.
+// ones, their probabilities, divided by their sum with `renorm`. Given experts outside [0, E) are refused.
 template <typename T, int NV>
 __global__ void __launch_bounds__(256) moe_gate_kernel(const T* logits, long long stride, int tokens, int E, int k,
                                                        int renorm, int given, long long* __restrict__ idx,
-                                                       float* __restrict__ weight) {
+                                                       float* __restrict__ weight, int* refused) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -293,10 +305,16 @@ __global__ void __launch_bounds__(256) moe_gate_kernel(const T* logits, long lon
   int my_e = 0;
   float my_w = 0.f, total = 0.f;
   if (given) {
-    if (lane < k) my_e = (int)idx[t * k + lane];
+    bool none = false;
+    if (lane < k) {
+      const long long e = idx[t * k + lane];
+      none = e < 0 || e >= E;
+      my_e = none ? -1 : (int)e;
+      if (none) refuse_expert(refused, e, t * k + lane, E);
+    }
     for (int j = 0; j < k; ++j) {
       const int e = __shfl_sync(0xffffffffu, my_e, j);
-      float own = 0.f;
+      float own = e < 0 ? __int_as_float(0x7fffffff) : 0.f;
 #pragma unroll
       for (int i = 0; i < NV; ++i)
         if (i * 32 + lane == e) own = s[i];
@@ -393,11 +411,13 @@ __global__ void __launch_bounds__(256) moe_gate_bwd_kernel(const T* __restrict__
 
 // Places of the pairs (token, slot) in the buffer sorted by expert, in the order of the pairs within an expert (deterministic). One
 // block per expert counts all pairs in shared memory (for the offsets) and ranks its own. dest[pair] = row, -1 for pairs of experts
-// outside [first, first + E); src[row] = pair, -1 for the rows that pad an expert's share to a multiple of 128.
+// outside [first, first + E), or -2 and refused if these experts are all the layer has (`whole`); src[row] = pair, -1 for the rows that
+// pad an expert's share to a multiple of 128.
 constexpr int MP_MAX_E = 2048, MP_THREADS = 1024;
 __global__ void __launch_bounds__(MP_THREADS) moe_place_kernel(const long long* idx, long long n, int first, int E,
                                                                int* __restrict__ dest, int* __restrict__ src,
-                                                               int* __restrict__ blk_expert, int nblk, int* __restrict__ expert_off) {
+                                                               int* __restrict__ blk_expert, int nblk, int* __restrict__ expert_off,
+                                                               int whole, int* refused) {
   __shared__ int hist[MP_MAX_E], off[MP_MAX_E + 1], part[2][32];
   pdl_trigger();
   pdl_wait();
@@ -407,7 +427,10 @@ __global__ void __launch_bounds__(MP_THREADS) moe_place_kernel(const long long* 
   for (long long i = tid; i < n; i += MP_THREADS) {
     const long long e = idx[i] - first;
     if (e >= 0 && e < E) atomicAdd(&hist[(int)e], 1);
-    else if (blockIdx.x == 0) dest[i] = -1;
+    else if (blockIdx.x == 0) {
+      dest[i] = whole ? -2 : -1;
+      if (whole) refuse_expert(refused, idx[i], i, E);
+    }
   }
   __syncthreads();
   padded_offsets(hist, off, E);
@@ -505,8 +528,8 @@ __global__ void __launch_bounds__(256) moe_rows_bwd_kernel(const __nv_bfloat16* 
   }
 }
 
-// y[t] = sum over the slots of w[t, j] * row[dest[t, j]] (w null: of the rows); pairs without a row count nothing. A block takes
-// 8 * blockDim elements of a token.
+// y[t] = sum over the slots of w[t, j] * row[dest[t, j]] (w null: of the rows); pairs without a row (-1) count nothing, a refused one
+// (-2) makes it no number. A block takes 8 * blockDim elements of a token.
 __global__ void __launch_bounds__(256) moe_weighted_sum_kernel(const __nv_bfloat16* row, const int* dest, const float* w, int k, int H,
                                                                __nv_bfloat16* __restrict__ y) {
   pdl_trigger();
@@ -518,7 +541,10 @@ __global__ void __launch_bounds__(256) moe_weighted_sum_kernel(const __nv_bfloat
 #pragma unroll 8
   for (int j = 0; j < k; ++j) {
     const int d = dest[t * k + j];
-    if (d < 0) continue;
+    if (d < 0) {
+      if (d == -2) a[0] = a[1] = a[2] = a[3] = a[4] = a[5] = a[6] = a[7] = __int_as_float(0x7fffffff);
+      continue;
+    }
     const float wj = w ? w[t * k + j] : 1.f;
     float f[8];
     ld8(row + (long long)d * H + v * 8, f);
@@ -608,18 +634,18 @@ extern "C" int vb_moe_sum(const void* out, const int* dest, const float* weight,
     else CALL(16);                \
   } while (0)
 
-// logits [T, stride] fp32 or bf16; idx int64 [T, k], read with `given`, written without; weight fp32 [T, k].
+// logits [T, stride] fp32 or bf16; idx int64 [T, k], read with `given`, written without; weight fp32 [T, k]; refused: refuse_expert.
 extern "C" int vb_moe_gate(const void* logits, long long stride, int T, int E, int k, int renorm, int given, int f32, long long* idx,
-                           float* weight, cudaStream_t stream) {
+                           float* weight, int* refused, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (E <= 0 || E > MR_MAX_E || k <= 0 || k > MR_MAX_TOP || k > E) return -3;
   const dim3 g((T + 7) / 8), b(256);
   cudaError_t e = cudaSuccess;
 #define VB_G(NV)                                                                                                                \
   e = f32 ? vb_launch_pdl(moe_gate_kernel<float, NV>, g, b, 0, stream, 1, (const float*)logits, stride, T, E, k, renorm, given, \
-                          idx, weight)                                                                                          \
+                          idx, weight, refused)                                                                                 \
           : vb_launch_pdl(moe_gate_kernel<bf16, NV>, g, b, 0, stream, 1, (const bf16*)logits, stride, T, E, k, renorm, given,   \
-                          idx, weight)
+                          idx, weight, refused)
   VB_GATE_NV(VB_G);
 #undef VB_G
   VB_DONE(e);
@@ -643,15 +669,15 @@ extern "C" int vb_moe_gate_bwd(const void* logits, long long stride, int T, int 
 }
 
 // idx int64 [n] expert of every pair; dest [n]; src [nblk * 128]; blk_expert [nblk]; expert_off [E + 1]. nblk * 128 rows have to be
-// enough for every expert's share rounded up to 128.
+// enough for every expert's share rounded up to 128. whole, refused: moe_place_kernel.
 extern "C" int vb_moe_place(const long long* idx, long long n, int first, int E, int* dest, int* src, int* blk_expert, int nblk,
-                            int* expert_off, cudaStream_t stream) {
+                            int* expert_off, int whole, int* refused, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (E <= 0 || E > MP_MAX_E || n > 0x7fffffffLL - 128ll * E ||
       (long long)nblk * MR_BLK + MR_BLK <= n + min((long long)E, n) * (MR_BLK - 1))
     return -3;
   VB_DONE(vb_launch_pdl(moe_place_kernel, dim3(E), dim3(MP_THREADS), 0, stream, 1, idx, n, first, E, dest, src, blk_expert, nblk,
-                        expert_off));
+                        expert_off, whole, refused));
 }
 
 extern "C" int vb_moe_rows(const void* x, const int* src, const int* blk_expert, long long rows, int k, int H, void* xs,

@@ -72,9 +72,9 @@ _SIGS = {
     "vb_moe_route": ([P, L, I, I, I, I, I, P, P, P, P, P, I, P, P], I),
     "vb_moe_gather": ([P, L, P, P, I, I, I, P, P, I, P], I),
     "vb_moe_sum": ([P, P, P, I, P, L, P, L, P, L, P, P, P, F, P, I, I, F, I, P], I),
-    "vb_moe_gate": ([P, L, I, I, I, I, I, I, P, P, P], I),
+    "vb_moe_gate": ([P, L, I, I, I, I, I, I, P, P, P, P], I),
     "vb_moe_gate_bwd": ([P, L, I, I, I, I, I, P, P, P, P, P], I),
-    "vb_moe_place": ([P, L, I, I, P, P, P, I, P, P], I),
+    "vb_moe_place": ([P, L, I, I, P, P, P, I, P, I, P, P], I),
     "vb_moe_rows": ([P, P, P, L, I, I, P, P], I),
     "vb_moe_rows_bwd": ([P, P, P, P, P, L, I, I, P, P, P], I),
     "vb_moe_weighted_sum": ([P, P, P, I, I, P, I, P], I),
@@ -241,3 +241,27 @@ def read_status(device=None) -> tuple[int, int, int]:
 
 def clear_status(device=None) -> None:
     status_word(device).zero_()
+
+
+_refused = None
+
+
+def refused_word() -> int | None:
+    """Address of four ints of host memory in which a kernel notes an index that it refuses. (None while a graph is captured and no
+    call before the capture has made them.)"""
+    global _refused
+    if _refused is None:
+        if torch.cuda.is_current_stream_capturing():
+            return None
+        words = torch.zeros(4, dtype=torch.int32, pin_memory=True)
+        _refused = words, (c_int * 4).from_address(words.data_ptr())
+    return _refused[0].data_ptr()
+
+
+def raise_refused() -> None:
+    """Raises, once, if a kernel that has run refused an index. Does not synchronise: like any error on the device, it is seen by the
+    first call that looks after the kernel."""
+    if _refused is not None and _refused[1][0]:
+        _, index, pair, bound = _refused[1]
+        _refused[1][0] = 0
+        raise NativeLibraryError(f"routed experts: index {index} of pair {pair} (token * slots + slot) is outside [0, {bound})")

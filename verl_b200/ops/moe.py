@@ -107,10 +107,11 @@ def moe_mlp(x: torch.Tensor, top_i: torch.Tensor, top_w: torch.Tensor, gate_up: 
     k = top_i.shape[1]
     E = gate_up.shape[0]
     if _fused_mlp_ok(x, top_i, top_w, gate_up, down, swiglu):
-        first = expert_offset if num_experts is not None and num_experts != E else 0
+        whole = num_experts is None or num_experts == E
+        first = 0 if whole else expert_offset
         if torch.is_grad_enabled() and any(t.requires_grad for t in (x, top_w, gate_up, down)):
-            return _RoutedMlpFn.apply(x, top_i, top_w, gate_up, down, first)
-        return _routed_mlp(x.contiguous(), top_i.contiguous(), top_w.contiguous(), gate_up, down, first)[0]
+            return _RoutedMlpFn.apply(x, top_i, top_w, gate_up, down, first, whole)
+        return _routed_mlp(x.contiguous(), top_i.contiguous(), top_w.contiguous(), gate_up, down, first, whole)[0]
     if num_experts is not None and num_experts != E:
         local = top_i - expert_offset
         local = torch.where((local >= 0) & (local < E), local, torch.full_like(local, E))
@@ -152,18 +153,21 @@ class _GateFn(torch.autograd.Function):
 
 
 def _gate(logits, k, renorm, given):
+    _lib.raise_refused()
     T, E = logits.shape
     idx = given if given is not None else torch.empty((T, k), dtype=torch.long, device=logits.device)
     w = torch.empty((T, k), dtype=torch.float32, device=logits.device)
     rc = _lib.fn("vb_moe_gate")(logits.data_ptr(), logits.stride(0), T, E, k, int(renorm), int(given is not None),
-                                int(logits.dtype == torch.float32), idx.data_ptr(), w.data_ptr(), _lib.stream())
+                                int(logits.dtype == torch.float32), idx.data_ptr(), w.data_ptr(), _lib.refused_word(), _lib.stream())
     _lib.check(rc, "vb_moe_gate")
     return idx, w
 
 
 def moe_gate(logits: torch.Tensor, k: int, renorm: bool, given: torch.Tensor | None = None):
     """Softmax gate: (weights fp32 [T, k], experts int64 [T, k]) of the ``k`` most probable experts of every row of ``logits``
-    [T, E], or of the ``given`` ones (router replay). ``renorm``: the weights are divided by their sum."""
+    [T, E], or of the ``given`` ones (router replay). ``renorm``: the weights are divided by their sum. A given expert outside [0, E) is
+    refused: on the host at once, on the device by ``_lib.raise_refused`` in the next call and in the optimizer step; its weight is no
+    number."""
     if (logits.is_cuda and logits.dtype in (torch.bfloat16, torch.float32) and logits.shape[1] <= 512 and k <= 32
             and logits.stride(1) == 1
             and (given is None or (given.dtype == torch.long and given.is_cuda and given.shape == (logits.shape[0], k)))):
@@ -192,9 +196,11 @@ def _fused_mlp_ok(x, top_i, top_w, gate_up, down, swiglu) -> bool:
             and gate_up.data_ptr() % 16 == 0 and down.data_ptr() % 16 == 0)
 
 
-def _routed_mlp(x, top_i, top_w, gate_up, down, first):
-    """x [T, H], top_i / top_w [T, k] contiguous, experts ``[first, first + E)`` -> (sum [T, H], what the backward needs).
+def _routed_mlp(x, top_i, top_w, gate_up, down, first, whole):
+    """x [T, H], top_i / top_w [T, k] contiguous, experts ``[first, first + E)`` -> (sum [T, H], what the backward needs). ``whole``:
+    these are all experts, others are refused as in :func:`moe_gate`; without it they are another rank's.
     Rows of blocks without an expert are never written; rows that pad an expert's share are zero in ``xs`` and so in ``h``."""
+    _lib.raise_refused()
     (T, H), k = x.shape, top_i.shape[1]
     E, I2, _ = gate_up.shape
     n, dev, stream = T * k, x.device, _lib.stream()
@@ -202,7 +208,7 @@ def _routed_mlp(x, top_i, top_w, gate_up, down, first):
     new = lambda *s, dt=torch.bfloat16: torch.empty(s, dtype=dt, device=dev)  # noqa: E731
     dest, src, blk, off = (new(m, dt=torch.int32) for m in (n, P, P // BLK, E + 1))
     rc = _lib.fn("vb_moe_place")(top_i.data_ptr(), n, first, E, dest.data_ptr(), src.data_ptr(), blk.data_ptr(), P // BLK,
-                                 off.data_ptr(), stream)
+                                 off.data_ptr(), int(whole), _lib.refused_word(), stream)
     _lib.check(rc, "vb_moe_place")
     xs = new(P, H)
     _lib.check(_lib.fn("vb_moe_rows")(x.data_ptr(), src.data_ptr(), blk.data_ptr(), P, k, H, xs.data_ptr(), stream), "vb_moe_rows")
@@ -219,9 +225,9 @@ class _RoutedMlpFn(torch.autograd.Function):
     """:func:`_routed_mlp` with gradients. If the stacked weights have ``main_grad`` (fp32), their gradients are accumulated there."""
 
     @staticmethod
-    def forward(ctx, x, top_i, top_w, gate_up, down, first):
+    def forward(ctx, x, top_i, top_w, gate_up, down, first, whole):
         x, top_i, top_w = x.contiguous(), top_i.contiguous(), top_w.contiguous()
-        y, kept = _routed_mlp(x, top_i, top_w, gate_up, down, first)
+        y, kept = _routed_mlp(x, top_i, top_w, gate_up, down, first, whole)
         ctx.save_for_backward(top_w, gate_up, down, *kept)
         return y
 
@@ -229,7 +235,7 @@ class _RoutedMlpFn(torch.autograd.Function):
     def backward(ctx, dy):
         top_w, gate_up, down, xs, gu, h, out, dest, src, blk, off = ctx.saved_tensors
         (T, k), (P, H), (E, I2, _) = top_w.shape, xs.shape, gate_up.shape
-        need_x, _, need_w, need_gu, need_down, _ = ctx.needs_input_grad
+        need_x, _, need_w, need_gu, need_down = ctx.needs_input_grad[:5]
         stream, dy = _lib.stream(), dy.contiguous()
         if dy.data_ptr() % 16:  # part of a larger gradient
             dy = dy.clone()
@@ -259,7 +265,7 @@ class _RoutedMlpFn(torch.autograd.Function):
                 _grouped(dgu, gate_up, dxs, P, H, I2, False, True, False, 1, E, blk, None)
                 rc = _lib.fn("vb_moe_weighted_sum")(dxs.data_ptr(), dest.data_ptr(), None, T, k, dx.data_ptr(), H, stream)
                 _lib.check(rc, "vb_moe_weighted_sum")
-        return dx, None, dw, d_gate_up, d_down, None
+        return dx, None, dw, d_gate_up, d_down, None, None
 
 
 # ----------------------------------------------------------------- inference: routing, experts and their sum as fused kernels

@@ -956,7 +956,9 @@ class NativeEngine(BaseEngine):
         """Global grad-norm, clip, fused AdamW on the shards. Returns the (pre-clip) gradient norm; a
         non-finite norm skips the update (verl/workers/actor/dp_actor.py:391-415)."""
         if self._lora_params:
-            return self._lora_optimizer_step()
+            norm = self._lora_optimizer_step()
+            ops._lib.raise_refused()
+            return norm
         z, oc = self.zero, self.optimizer_config
         clip = float(_cfg(oc, "clip_grad", 1.0) if self.clip_grad_override is None else self.clip_grad_override)
         lr = self._lr()
@@ -1009,6 +1011,7 @@ class NativeEngine(BaseEngine):
             z.master[a:b].copy_(saved)
             z.shard16[a:b].copy_(saved.to(z.shard16.dtype))
         z.zero_grad()
+        ops._lib.raise_refused()  # the norm has been waited for: whatever the step's kernels refused is known
         return norm
 
     _TP_SLICED = ("qkv_proj.weight", "qkv_proj.bias", "gate_up_proj.weight", "o_proj.weight", "down_proj.weight",

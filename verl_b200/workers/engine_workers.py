@@ -23,6 +23,7 @@ import torch.distributed as dist
 
 from ..models import CausalLM, ModelConfig, build_model, preset
 from ..models.hf_io import load_hf_checkpoint
+from ..ops._lib import raise_refused
 from ..protocol import DataProto
 from ..single_controller.base import Dispatch, Worker, register
 from ..single_controller.base.decorator import make_nd_compute_dataproto_dispatch_fn
@@ -438,6 +439,7 @@ class ActorRolloutRefWorker(_WorkerBase):
         with self.actor_engine.eval_mode():
             lp, ent = self.actor.compute_log_prob(data, calculate_entropy=True)
         tensors = {"old_log_probs": lp.cpu(), "entropys": ent.cpu()}
+        raise_refused()  # replayed experts that the model does not have
         if self.actor.last_routed_experts is not None:  # router replay R2: the experts this pass routed every token to
             tensors["routed_experts"] = self.actor.last_routed_experts
         if self.actor.last_sum_pi_squared is not None:  # actor.calculate_sum_pi_squared (optimal token baseline)
