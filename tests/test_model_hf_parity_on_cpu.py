@@ -65,3 +65,40 @@ def test_fused_logprob_matches_logits_path():
     torch.testing.assert_close(lp, ref, atol=1e-5, rtol=1e-5)
     p = torch.softmax(logits, -1)
     torch.testing.assert_close(ent, -(p * torch.log(p)).sum(-1), atol=1e-4, rtol=1e-4)
+
+
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("how", ["hook", "pre_hook", "forward", "subclass", "global"])
+def test_gate_up_module_is_called_where_it_is_not_a_plain_product(how, grad):
+    """Hooks, a forward of its own and subclasses of the gate | up projection take part in the MLP, with and without gradients."""
+    from verl_b200.models.transformer import DenseMLP, Linear
+
+    torch.manual_seed(1)
+    mlp = DenseMLP(preset("tiny-qwen2"), torch.float32, "cpu")
+    for p in mlp.parameters():
+        torch.nn.init.normal_(p, 0.0, 0.05)
+    x = torch.randn(5, mlp.gate_up_proj.weight.shape[1])
+    m, handle = mlp.gate_up_proj, None
+    if how == "hook":
+        m.register_forward_hook(lambda mod, args, out: 2 * out)
+    elif how == "pre_hook":
+        m.register_forward_pre_hook(lambda mod, args: (2 * args[0],))
+    elif how == "forward":
+        plain = m.forward
+        m.forward = lambda v: 2 * plain(v)
+    elif how == "subclass":
+        class Twice(Linear):
+            def forward(self, v):
+                return 2 * super().forward(v)
+
+        m.__class__ = Twice
+    else:
+        handle = torch.nn.modules.module.register_module_forward_hook(lambda mod, args, out: 2 * out if mod is m else out)
+    try:
+        with torch.set_grad_enabled(grad):
+            got = mlp(x)
+    finally:
+        if handle is not None:
+            handle.remove()
+    g, u = (2 * (x @ m.weight.detach().t())).chunk(2, -1)
+    torch.testing.assert_close(got.detach(), (torch.nn.functional.silu(g) * u) @ mlp.down_proj.weight.detach().t())

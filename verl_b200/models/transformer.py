@@ -94,6 +94,17 @@ class Linear(nn.Module):
         return y
 
 
+    def is_own(self) -> bool:
+        """A call runs this class's forward and nothing else (no hook, replaced forward or subclass), so nobody else holds its result."""
+        return (type(self) is Linear and "forward" not in self.__dict__
+                and not (self._forward_hooks or self._forward_pre_hooks or self._backward_hooks or self._backward_pre_hooks
+                         or nn.modules.module._has_any_global_hook()))
+
+    def is_product(self) -> bool:
+        """A call is the matrix product and nothing else: a kernel that takes the weight may stand for it."""
+        return self.is_own() and self.bias is None and "lora_A" not in self.__dict__
+
+
 class RMSNormWeight(nn.Module):
     def __init__(self, dim: int, dtype, device):
         super().__init__()
@@ -114,7 +125,7 @@ class DenseMLP(nn.Module):
 
             x = copy_to_tp_region(x, self.tp_group)
             return reduce_from_tp_region(self.down_proj(ops.swiglu(self.gate_up_proj(x))), self.tp_group)
-        if "lora_A" not in self.gate_up_proj.__dict__ and self.gate_up_proj.bias is None:
+        if isinstance(self.gate_up_proj, Linear) and self.gate_up_proj.is_product():
             return self.down_proj(ops.linear_swiglu(x, self.gate_up_proj.weight))
         return self.down_proj(ops.swiglu(self.gate_up_proj(x)))
 
