@@ -584,6 +584,23 @@ def test_paged_decode_attention(B, Hq, Hk, D, bs, maxlen):
             _bf16_close(out, ref, ulps=4)
 
 
+def test_hooked_projection_keeps_its_result():
+    """A forward hook on the projection of a layer with head norms may keep what it is given: the pass without gradients does not write
+    over it, and gives the bits that it gives without the hook."""
+    from verl_b200.models import PackedBatch, build_model, preset
+
+    model = build_model(preset("tiny-qwen2", model_type="qwen3", head_dim=64), device="cuda")
+    ids = torch.arange(3, 40, device="cuda")
+    batch = PackedBatch(ids, torch.arange(37, device="cuda"), torch.tensor([0, 37], dtype=torch.int32, device="cuda"), 37)
+    kept = []
+    with torch.no_grad():
+        want = model.forward_hidden(batch)
+        handle = model.layers[0].self_attn.qkv_proj.register_forward_hook(lambda m, a, out: kept.append((out, out.clone())) or None)
+        got = model.forward_hidden(batch)
+        handle.remove()
+    assert len(kept) == 1 and torch.equal(*kept[0]) and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("Hq,Hk,D,bs,lens", [(14, 2, 64, 16, (500, 1, 129)), (8, 8, 64, 8, (3000, 17)), (32, 2, 64, 32, (700, 64)),
                                              (8, 1, 128, 256, (2100, 255, 300)), (9, 1, 128, 512, (513, 30))])
 def test_decode_attention_weights_stay_in_fp32(Hq, Hk, D, bs, lens):

@@ -326,7 +326,9 @@ class Attention(nn.Module):
             norms = self.q_norm.weight, self.k_norm.weight
             if self.tp_group is not None:  # shared by all heads: every rank sees its own heads' share of the gradient
                 norms = tuple(copy_to_tp_region(w, self.tp_group) for w in norms)
-        heads = ops.qkv_heads(qkv, batch.position_ids, rope[0], rope[1], Hq, Hk, D, norms, cfg.rms_norm_eps)
+        # without norms the projection is rotated in place by rope_qkv, too; before norms it is kept for whoever else may hold it
+        own = norms is None or (isinstance(self.qkv_proj, Linear) and self.qkv_proj.is_own())
+        heads = ops.qkv_heads(qkv, batch.position_ids, rope[0], rope[1], Hq, Hk, D, norms, cfg.rms_norm_eps, in_place=own)
         if heads is None:
             if norms is not None:
                 q, k, v = qkv.split([cfg.q_size, cfg.kv_size, cfg.kv_size], dim=-1)

@@ -309,18 +309,19 @@ class _QkvFn(torch.autograd.Function):
 
 
 def qkv_heads(qkv: torch.Tensor, pos: torch.Tensor, cos_t: torch.Tensor, sin_t: torch.Tensor, Hq: int, Hk: int, D: int,
-              norms: tuple | None, eps: float):
-    """q [T, Hq, D], k and v [T, Hk, D] of a packed projection ``qkv`` [T, (Hq + 2 Hk) * D] that nothing else reads, after head norms
-    (``norms``: weights of q and of k, or None) and rotate-half positions; forward and backward are one pass each. None where that does
-    not apply: host tensors, other sizes or types, multimodal positions."""
+              norms: tuple | None, eps: float, in_place: bool = True):
+    """q [T, Hq, D], k and v [T, Hk, D] of a packed projection ``qkv`` [T, (Hq + 2 Hk) * D] after head norms (``norms``: weights of q and
+    of k, or None) and rotate-half positions; forward and backward are one pass each. ``in_place``: nothing else reads ``qkv``, and the
+    result may take its memory. None where that does not apply: host tensors, other sizes or types, multimodal positions."""
     if not _head_norm_rope_ok(qkv, pos, cos_t, sin_t, D, norms):
         return None
     pos, (qw, kw) = pos.contiguous(), norms or (None, None)
     if not _lib.plain():
         return _QkvFn.apply(qkv, qw, kw, pos, cos_t, sin_t, Hq, Hk, D, eps)
-    _head_norm_rope(qkv, qkv, pos, cos_t, sin_t, Hq, Hk, D, norms, eps)
+    out = qkv if in_place else torch.empty_like(qkv, memory_format=torch.contiguous_format)
+    _head_norm_rope(qkv, out, pos, cos_t, sin_t, Hq, Hk, D, norms, eps)
     T, nq, nk = qkv.shape[0], Hq * D, Hk * D
-    return qkv[:, :nq].view(T, Hq, D), qkv[:, nq : nq + nk].view(T, Hk, D), qkv[:, nq + nk :].view(T, Hk, D)
+    return out[:, :nq].view(T, Hq, D), out[:, nq : nq + nk].view(T, Hk, D), out[:, nq + nk :].view(T, Hk, D)
 
 
 def head_norm_rope_kv_write(qkv: torch.Tensor, q_weight: torch.Tensor | None, k_weight: torch.Tensor | None,
