@@ -4,6 +4,8 @@ and the native sources carry a binding for every exported entry point that Pytho
 import importlib
 import pkgutil
 import re
+import subprocess
+import sys
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent.parent
@@ -70,3 +72,16 @@ def test_kernels_that_start_early_use_no_read_only_loads():
                 assert "asm volatile" in body and '"memory"' in body
             found += [(name, w) for w in ("__ldg(", "ld.global.nc") if w in body]
     assert seen >= 12 and not found, (seen, found)
+
+
+def test_imports_with_a_torch_that_has_no_cuda():
+    code = """
+import torch
+for name in [n for n in vars(torch._C) if n.startswith("_cuda_")]:
+    delattr(torch._C, name)
+import verl_b200.ops, verl_b200.models
+x = torch.randn(3, 8)
+assert torch.equal(verl_b200.ops.swiglu(x), torch.nn.functional.silu(x[:, :4]) * x[:, 4:])
+"""
+    done = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]

@@ -19,7 +19,8 @@ from torch.autograd import forward_ad as _forward_ad
 _LIB = None
 _LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libverl_b200.so"
 
-_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+# builds of torch without CUDA have neither
+_raw_stream, _current_device = (getattr(torch._C, name, None) for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
 
 P, I, L, F, U = c_void_p, c_int, c_longlong, c_float, c_ulonglong
 
@@ -199,6 +200,8 @@ def ptr(t) -> int | None:
 def stream() -> int:
     """The current stream of the current device, without the stream object that ``torch.cuda.current_stream`` builds (7 us a call,
     a fifth of the host time of a forward on short sequences; 0.3 us this way)."""
+    if _raw_stream is None or _current_device is None:
+        return torch.cuda.current_stream().cuda_stream
     return _raw_stream(_current_device())
 
 
