@@ -891,6 +891,39 @@ def test_experts_outside_the_layer_are_refused(bad, renorm):
     assert not bool(part.isnan().any())
 
 
+def test_traces_and_forward_mode_pass_through():
+    """A trace of an op without gradients computes new inputs, and a tangent of the routing weights reaches the routed sum, as
+    through torch's own operators."""
+    from torch.autograd import forward_ad
+
+    from verl_b200 import ops
+    from verl_b200.ops.moe import moe_gate, moe_mlp
+
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    T, E, k, H, I = 24, 4, 2, 64, 64
+    w, wn = rnd(2 * I, H).bfloat16() * 0.1, rnd(H).bfloat16()
+    gate_up, down = (rnd(*s).bfloat16() * 0.1 for s in ((E, 2 * I, H), (E, H, I)))
+    x, x2 = rnd(T, H).bfloat16(), rnd(T, H).bfloat16()
+    router = rnd(E, H).bfloat16() * 0.1
+
+    with torch.no_grad():
+        p, idx = moe_gate(rnd(T, E), k, True)
+        for op in (lambda v: ops.rmsnorm(v, wn)[0], lambda v: ops.linear(v, w), lambda v: ops.linear_swiglu(v, w), ops.swiglu,
+                   lambda v: moe_gate(ops.linear(v, router), k, True)[0], lambda v: moe_mlp(v, idx, p, gate_up, down, ops.swiglu)):
+            _bf16_close(torch.jit.trace(op, x, check_trace=False)(x2), op(x2), ulps=4)
+        dp = rnd(T, k)
+        with forward_ad.dual_level():
+            y = moe_mlp(x, idx, forward_ad.make_dual(p, dp), gate_up, down, ops.swiglu)
+            tangent = forward_ad.unpack_dual(y).tangent
+            z = forward_ad.make_dual(rnd(T, E), rnd(T, E))
+            assert forward_ad.unpack_dual(moe_gate(z, k, True)[0]).tangent is not None
+        assert tangent is not None
+        # the sum is linear in the weights: two bf16 roundings of the terms and one of the sum
+        want = moe_mlp(x, idx, dp, gate_up, down, ops.swiglu).double()
+        assert float((tangent.double() - want).abs().max()) <= 3 * 2.0 ** -8 * float(want.abs().max())
+
+
 def test_bounded_device_wait_reports_status_and_context_survives():
     """A cross-rank barrier whose peer never arrives: the kernel gives up after its time limit, records the wait in
     the status word and returns; the host reads the code and the context keeps working."""

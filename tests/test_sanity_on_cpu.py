@@ -85,3 +85,20 @@ assert torch.equal(verl_b200.ops.swiglu(x), torch.nn.functional.silu(x[:, :4]) *
 """
     done = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert done.returncode == 0, done.stderr[-2000:]
+
+
+def test_short_cuts_are_off_where_something_follows_the_computation():
+    import torch
+    from torch.autograd import forward_ad
+
+    from verl_b200.ops import _lib
+
+    assert not _lib.plain() and not _lib.followed()
+    seen = []
+    with torch.no_grad():
+        assert _lib.plain()
+        torch.jit.trace(lambda x: (seen.append((_lib.plain(), _lib.followed())), x + 1)[1], torch.ones(2), check_trace=False)
+        with forward_ad.dual_level():
+            seen.append((_lib.plain(), _lib.followed()))
+        assert _lib.plain()
+    assert seen == [(False, True), (False, True)]

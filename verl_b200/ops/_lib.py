@@ -205,10 +205,16 @@ def stream() -> int:
     return _raw_stream(_current_device())
 
 
+def followed() -> bool:
+    """Something else than the backward follows what is computed, through torch's own operators and autograd functions: a forward-mode
+    level, or a trace (which would keep the empty result of a native call as a constant)."""
+    return _forward_ad._current_level >= 0 or torch.jit.is_tracing()
+
+
 def plain() -> bool:
-    """Nothing records what is computed: no gradients, no forward-mode level. An autograd function's forward is then its result, and
-    going through ``Function.apply`` only costs (5 us a call)."""
-    return not torch.is_grad_enabled() and _forward_ad._current_level < 0
+    """Nothing records what is computed: no gradients, no forward-mode level, no trace. An autograd function's forward is then its
+    result, and going through ``Function.apply`` only costs (5 us a call)."""
+    return not torch.is_grad_enabled() and not followed()
 
 
 def check(rc: int, what: str) -> None:

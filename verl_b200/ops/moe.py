@@ -169,7 +169,7 @@ def moe_gate(logits: torch.Tensor, k: int, renorm: bool, given: torch.Tensor | N
     refused: on the host at once, on the device by ``_lib.raise_refused`` in the next call and in the optimizer step; its weight is no
     number."""
     if (logits.is_cuda and logits.dtype in (torch.bfloat16, torch.float32) and logits.shape[1] <= 512 and k <= 32
-            and logits.stride(1) == 1
+            and logits.stride(1) == 1 and not _lib.followed()
             and (given is None or (given.dtype == torch.long and given.is_cuda and given.shape == (logits.shape[0], k)))):
         if given is not None:
             given = given.contiguous()
@@ -189,7 +189,7 @@ def _fused_mlp_ok(x, top_i, top_w, gate_up, down, swiglu) -> bool:
     from . import nn
 
     H, I2 = x.shape[1], gate_up.shape[1]
-    return (x.is_cuda and swiglu is nn.swiglu and x.shape[0] > 0 and x.dtype == gate_up.dtype == down.dtype == torch.bfloat16
+    return (x.is_cuda and swiglu is nn.swiglu and not _lib.followed() and x.shape[0] > 0 and x.dtype == gate_up.dtype == down.dtype == torch.bfloat16
             and x.data_ptr() % 16 == 0 and top_i.shape == top_w.shape and top_i.shape[0] == x.shape[0]
             and top_i.dtype == torch.long and top_w.dtype == torch.float32 and gate_up.shape[0] <= 2048 and H % 64 == 0
             and I2 % 128 == 0 and gate_up.is_contiguous() and down.is_contiguous()
