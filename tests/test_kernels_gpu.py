@@ -891,6 +891,42 @@ def test_experts_outside_the_layer_are_refused(bad, renorm):
     assert not bool(part.isnan().any())
 
 
+@pytest.mark.parametrize("renorm", [True, False])
+def test_second_derivatives_of_gate_and_routed_sum(renorm):
+    """Gradients taken with ``create_graph`` are those of the kernels, and differentiating them gives what torch gives in fp64 (gate: all
+    second derivatives; routed sum: those by the routing weights, its products have a first backward only)."""
+    from verl_b200 import ops
+    from verl_b200.ops.moe import moe_gate, moe_mlp
+
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    T, E, k, H, I = 20, 8, 2, 64, 64
+    z, g = rnd(T, E).requires_grad_(True), rnd(T, k).requires_grad_(True)
+    w, idx = moe_gate(z, k, renorm)
+    (dz,) = torch.autograd.grad(w, z, g, create_graph=True)
+    assert float((dz - torch.autograd.grad(w, z, g, retain_graph=True)[0]).abs().max()) < 1e-6
+    v = rnd(T, E)
+    got = torch.autograd.grad(dz, (z, g), v)
+    zr, gr = z.detach().double().requires_grad_(True), g.detach().double().requires_grad_(True)
+    p = torch.softmax(zr, -1).gather(1, idx)
+    p = p / p.sum(-1, keepdim=True) if renorm else p
+    (dzr,) = torch.autograd.grad(p, zr, gr, create_graph=True)
+    for a, b in zip(got, torch.autograd.grad(dzr, (zr, gr), v.double())):
+        assert float((a.double() - b).abs().max()) <= 64 * 2.0 ** -24 * max(1.0, float(b.abs().max()))
+    gate_up, down = (rnd(*s).bfloat16() * 0.1 for s in ((E, 2 * I, H), (E, H, I)))
+    x, dy = rnd(T, H).bfloat16(), rnd(T, H).bfloat16().requires_grad_(True)
+    top_w = w.detach().t().contiguous().t().requires_grad_(True)  # not contiguous
+    y = moe_mlp(x, idx, top_w, gate_up, down, ops.swiglu)
+    (first,) = torch.autograd.grad(y, top_w, dy, create_graph=True)
+    (plain,) = torch.autograd.grad(y, top_w, dy.detach(), retain_graph=True)
+    scale = float(plain.abs().max())
+    assert float((first - plain).abs().max()) <= 4 * 2.0 ** -8 * scale  # bf16 terms, summed
+    (back,) = torch.autograd.grad(first, dy, torch.ones_like(first))
+    # linear in dy: the sum of the experts' rows, weights 1
+    want = moe_mlp(x, idx, torch.ones_like(top_w), gate_up, down, ops.swiglu).double()
+    assert float((back.double() - want).abs().max()) <= 4 * 2.0 ** -8 * float(want.abs().max())
+
+
 def test_traces_and_forward_mode_pass_through():
     """A trace of an op without gradients computes new inputs, and a tangent of the routing weights reaches the routed sum, as
     through torch's own operators."""
@@ -911,7 +947,9 @@ def test_traces_and_forward_mode_pass_through():
         p, idx = moe_gate(rnd(T, E), k, True)
         for op in (lambda v: ops.rmsnorm(v, wn)[0], lambda v: ops.linear(v, w), lambda v: ops.linear_swiglu(v, w), ops.swiglu,
                    lambda v: moe_gate(ops.linear(v, router), k, True)[0], lambda v: moe_mlp(v, idx, p, gate_up, down, ops.swiglu)):
-            _bf16_close(torch.jit.trace(op, x, check_trace=False)(x2), op(x2), ulps=4)
+            got, want = torch.jit.trace(op, x, check_trace=False)(x2).double(), op(x2).double()
+            # the routed sum has its terms and its sum in bf16 then, 2^-9 each of the largest
+            assert float((got - want).abs().max()) <= 4 * 2.0 ** -9 * float(want.abs().max())
         dp = rnd(T, k)
         with forward_ad.dual_level():
             y = moe_mlp(x, idx, forward_ad.make_dual(p, dp), gate_up, down, ops.swiglu)

@@ -103,8 +103,6 @@ def moe_mlp(x: torch.Tensor, top_i: torch.Tensor, top_w: torch.Tensor, gate_up: 
     Expert parallelism over replicated tokens: with ``num_experts`` larger than ``E`` the matrices are the experts
     ``[expert_offset, expert_offset + E)`` of the layer; pairs routed elsewhere fall into a spare bucket whose blocks
     the grouped GEMM skips, and the result is this rank's partial sum (the ranks' results add up to the layer's)."""
-    T, H = x.shape
-    k = top_i.shape[1]
     E = gate_up.shape[0]
     if _fused_mlp_ok(x, top_i, top_w, gate_up, down, swiglu):
         whole = num_experts is None or num_experts == E
@@ -112,6 +110,12 @@ def moe_mlp(x: torch.Tensor, top_i: torch.Tensor, top_w: torch.Tensor, gate_up: 
         if torch.is_grad_enabled() and any(t.requires_grad for t in (x, top_w, gate_up, down)):
             return _RoutedMlpFn.apply(x, top_i, top_w, gate_up, down, first, whole)
         return _routed_mlp(x.contiguous(), top_i.contiguous(), top_w.contiguous(), gate_up, down, first, whole)[0]
+    return _general_mlp(x, top_i, top_w, gate_up, down, swiglu, expert_offset, num_experts)
+
+
+def _general_mlp(x, top_i, top_w, gate_up, down, swiglu, expert_offset, num_experts):
+    """:func:`moe_mlp` of any sizes and types, by torch's operators around the grouped products."""
+    (T, H), k, E = x.shape, top_i.shape[1], gate_up.shape[0]
     if num_experts is not None and num_experts != E:
         local = top_i - expert_offset
         local = torch.where((local >= 0) & (local < E), local, torch.full_like(local, E))
@@ -142,6 +146,8 @@ class _GateFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g, _):
         logits, idx, w = ctx.saved_tensors
+        if torch.is_grad_enabled():  # the gradient is differentiated itself
+            return torch.autograd.grad(_gate_weights(logits, idx, ctx.renorm), logits, g, create_graph=True) + (None,) * 3
         (T, E), k = logits.shape, idx.shape[1]
         dz = torch.empty((T, E), dtype=logits.dtype, device=logits.device)
         g = g.contiguous()
@@ -150,6 +156,11 @@ class _GateFn(torch.autograd.Function):
                                         dz.data_ptr(), _lib.stream())
         _lib.check(rc, "vb_moe_gate_bwd")
         return dz, None, None, None
+
+
+def _gate_weights(logits, idx, renorm):
+    w = torch.softmax(logits.float(), dim=-1).gather(-1, idx)
+    return w / w.sum(-1, keepdim=True) if renorm else w
 
 
 def _gate(logits, k, renorm, given):
@@ -177,11 +188,9 @@ def moe_gate(logits: torch.Tensor, k: int, renorm: bool, given: torch.Tensor | N
             return _GateFn.apply(logits, k, renorm, given)
         idx, w = _gate(logits, k, renorm, given)
         return w, idx
-    probs = torch.softmax(logits.float(), dim=-1)
     if given is not None:
-        top_i, top_w = given, probs.gather(-1, given)
-    else:
-        top_w, top_i = torch.topk(probs, k, dim=-1)
+        return _gate_weights(logits, given, renorm), given
+    top_w, top_i = torch.topk(torch.softmax(logits.float(), dim=-1), k, dim=-1)
     return (top_w / top_w.sum(-1, keepdim=True) if renorm else top_w), top_i
 
 
@@ -221,22 +230,36 @@ def _routed_mlp(x, top_i, top_w, gate_up, down, first, whole):
     return y, (xs, gu, h, out, dest, src, blk, off)
 
 
+def _differentiable_mlp_grads(ctx, dy, x, top_i, top_w, gate_up, down):
+    from . import nn
+
+    inputs = (x, None, top_w, gate_up, down)
+    y = _general_mlp(x, top_i, top_w, gate_up, down, nn.swiglu, *ctx.experts)
+    asked = [i for i, t in enumerate(inputs) if t is not None and ctx.needs_input_grad[i]]
+    grads = [None] * 7
+    for i, g in zip(asked, torch.autograd.grad(y, [inputs[i] for i in asked], dy, create_graph=True, allow_unused=True)):
+        grads[i] = g
+    return tuple(grads)
+
+
 class _RoutedMlpFn(torch.autograd.Function):
     """:func:`_routed_mlp` with gradients. If the stacked weights have ``main_grad`` (fp32), their gradients are accumulated there."""
 
     @staticmethod
     def forward(ctx, x, top_i, top_w, gate_up, down, first, whole):
-        x, top_i, top_w = x.contiguous(), top_i.contiguous(), top_w.contiguous()
-        y, kept = _routed_mlp(x, top_i, top_w, gate_up, down, first, whole)
-        ctx.save_for_backward(top_w, gate_up, down, *kept)
+        y, kept = _routed_mlp(x.contiguous(), top_i.contiguous(), top_w.contiguous(), gate_up, down, first, whole)
+        ctx.save_for_backward(x, top_i, top_w, gate_up, down, *kept)
+        ctx.experts = first, None if whole else -1  # as _general_mlp takes them
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        top_w, gate_up, down, xs, gu, h, out, dest, src, blk, off = ctx.saved_tensors
+        x, top_i, top_w, gate_up, down, xs, gu, h, out, dest, src, blk, off = ctx.saved_tensors
+        if torch.is_grad_enabled():  # the gradient is differentiated itself
+            return _differentiable_mlp_grads(ctx, dy, x, top_i, top_w, gate_up, down)
         (T, k), (P, H), (E, I2, _) = top_w.shape, xs.shape, gate_up.shape
         need_x, _, need_w, need_gu, need_down = ctx.needs_input_grad[:5]
-        stream, dy = _lib.stream(), dy.contiguous()
+        stream, dy, top_w = _lib.stream(), dy.contiguous(), top_w.contiguous()
         if dy.data_ptr() % 16:  # part of a larger gradient
             dy = dy.clone()
         new = lambda *s: torch.empty(s, dtype=torch.bfloat16, device=dy.device)  # noqa: E731
