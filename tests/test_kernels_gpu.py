@@ -468,6 +468,36 @@ def test_sampler_never_takes_a_token_of_no_weight():
     assert bool((tok == 77).all())
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_position_tables_off_a_16_byte_boundary(D):
+    """They are read 16 bytes at a time: tables that lie 4 bytes off take the separate steps, which give the same bits, and the kernel's
+    entry points refuse them."""
+    from verl_b200 import ops
+    from verl_b200.ops import _lib
+
+    T, Hq, Hk = 9, 4, 2
+    qkv = torch.randn(T, (Hq + 2 * Hk) * D, device="cuda").bfloat16()
+    pos = torch.arange(T, device="cuda")
+    tables = ops.rope_tables(D, 64, 10000.0, "cuda")
+    off = []
+    for t in tables:
+        off.append(torch.empty(t.numel() + 1, device="cuda")[1:].view(t.shape))
+        off[-1].copy_(t)
+    with torch.no_grad():
+        want = ops.rope_qkv(qkv.clone(), pos, *tables, Hq, Hk, D)
+        assert ops.qkv_heads(qkv.clone(), pos, *off, Hq, Hk, D, None, 1e-6) is None
+        assert not ops.head_norm_rope_(qkv.clone(), pos, *off, Hq, Hk, D, None, 1e-6)
+        assert torch.equal(ops.rope_qkv(qkv.clone(), pos, *off, Hq, Hk, D), want)
+        q, _, _ = ops.qkv_heads(qkv.clone(), pos, *tables, Hq, Hk, D, None, 1e-6)
+        assert torch.equal(q.reshape(T, -1), want[:, : Hq * D])
+    out = torch.empty_like(qkv)
+    head = (qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), pos.data_ptr())
+    tail = (None, None, 1e-6, T, Hq, Hk, D)
+    assert _lib.fn("vb_head_norm_rope")(*head, off[0].data_ptr(), off[1].data_ptr(), *tail, None, None, None, 0, _lib.stream()) == -3
+    assert _lib.fn("vb_head_norm_rope_bwd")(*(qkv.data_ptr(),) * 3, None, 0, pos.data_ptr(), off[0].data_ptr(), off[1].data_ptr(), *tail,
+                                            out.data_ptr(), None, None, None, 0, 0, _lib.stream()) == -3
+
+
 @pytest.mark.parametrize("T,Hq,Hk,D,bs", [(1, 14, 2, 64, 16), (37, 28, 4, 128, 16), (5, 3, 1, 256, 8), (129, 9, 3, 64, 64)])
 @pytest.mark.parametrize("norm", [False, True])
 def test_head_norm_rope(T, Hq, Hk, D, bs, norm):

@@ -594,13 +594,15 @@ extern "C" int vb_rope(void* q, void* k, long long q_stride, long long k_stride,
   return rope_launch(q, k, q_stride, k_stride, pos, cos_t, sin_t, T, Hq, Hk, D, backward, 0, 0, stream);
 }
 
-// D 64, 128 or 256; rows, results and caches on 8-byte boundaries. qw and kw both or neither.
+// D 64, 128 or 256; rows, results, caches and norms on 8-byte boundaries, tables on 16-byte ones. qw and kw both or neither.
 extern "C" int vb_head_norm_rope(const void* qkv, long long stride, void* out, long long out_stride, const long long* pos,
                                  const float* cos_t, const float* sin_t, const void* qw, const void* kw, float eps, long long T, int Hq,
                                  int Hk, int D, const long long* slots, void* kc, void* vc, int block_size, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (((stride | out_stride) & 3) || ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 7) ||
       (qw == nullptr) != (kw == nullptr) ||
+      ((reinterpret_cast<uintptr_t>(qw) | reinterpret_cast<uintptr_t>(kw)) & 7) ||
+      ((reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15) ||
       (slots && (((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 7) || block_size <= 0)))
     return -3;
   const long long threads = T * (Hq + Hk + (slots || out != qkv ? Hk : 0)) * (D / 8), blocks = (threads + 255) / 256;
@@ -619,7 +621,7 @@ extern "C" int vb_head_norm_rope(const void* qkv, long long stride, void* out, l
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
-// dq, dk, dv, dqkv contiguous and on 8-byte boundaries. With norms: x the projection, part fp32 [2, parts, D], dqw and dkw fp32 [D]
+// dq, dk, dv, dqkv contiguous and on 8-byte boundaries, norms and tables as above. With norms: x the projection, part fp32 [2, parts, D], dqw and dkw fp32 [D]
 // (accumulate: added to).
 extern "C" int vb_head_norm_rope_bwd_parts() { return 4 * vb_num_sms(); }
 extern "C" int vb_head_norm_rope_bwd(const void* dq, const void* dk, const void* dv, const void* x, long long x_stride,
@@ -629,7 +631,10 @@ extern "C" int vb_head_norm_rope_bwd(const void* dq, const void* dk, const void*
   if (T <= 0) return 0;
   const uintptr_t at = reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv) |
                        reinterpret_cast<uintptr_t>(dqkv) | (qw ? reinterpret_cast<uintptr_t>(x) : 0);
-  if ((at & 7) || (qw && ((x_stride & 3) || !kw || !part || !dqw || !dkw))) return -3;
+  if ((at & 7) || (qw && ((x_stride & 3) || !kw || !part || !dqw || !dkw)) ||
+      ((reinterpret_cast<uintptr_t>(qw) | reinterpret_cast<uintptr_t>(kw)) & 7) ||
+      ((reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t)) & 15))
+    return -3;
   const int parts = vb_head_norm_rope_bwd_parts();
 #define VB_HNRB(DD)                                                                                                                \
   head_norm_rope_bwd_kernel<DD><<<parts, 256, 0, stream>>>((const __nv_bfloat16*)dq, (const __nv_bfloat16*)dk, (const __nv_bfloat16*)dv, \

@@ -246,7 +246,8 @@ def rotate_pairs(x: torch.Tensor, positions: torch.Tensor, freqs: torch.Tensor, 
 def _head_norm_rope_ok(qkv, pos, cos_t, sin_t, D, norms) -> bool:
     return (qkv.is_cuda and qkv.dtype == torch.bfloat16 and D in (64, 128, 256) and pos.dim() == 1 and pos.dtype == torch.long
             and qkv.dim() == 2 and qkv.stride(1) == 1 and qkv.stride(0) % 4 == 0 and qkv.data_ptr() % 8 == 0
-            and cos_t.shape[1] == D // 2 and cos_t.is_contiguous() and sin_t.is_contiguous()
+            and cos_t.shape[1] == D // 2 and cos_t.dtype == sin_t.dtype == torch.float32 and cos_t.is_contiguous()
+            and sin_t.is_contiguous() and (cos_t.data_ptr() | sin_t.data_ptr()) % 16 == 0
             and all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.data_ptr() % 8 == 0 for w in norms or ()))
 
 
