@@ -127,12 +127,14 @@ using namespace vb;
 //   3584 -> 37888  45 / 59 / 67 / 81 (66 / 52 / 46 / 46)  18944 -> 3584  23 / 27 / 32 / 40 (30 to 38)
 // Beyond 8 rows the loads of A (from L2, by every block) grow to those of B: where tiles of the tcgen05 kernel fill all SMs it is as
 // fast at 16 rows and faster beyond, and with long rows (K) its staged operands win from 24 and 32 rows on.
-bool vb_gemm_skinny_ok(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb) {
-  const uintptr_t at = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B);
-  if ((K & 7) || (lda & 7) || (ldb & 7) || (at & 15)) return false;
+bool vb_gemm_skinny_rows(int M, int N, int K) {
   if (M <= 8) return true;
   if (N >= 256 * vb_num_sms()) return false;
   return M <= 16 || (M <= 24 && K <= 8192) || (M <= 32 && K <= 4096);
+}
+bool vb_gemm_skinny_ok(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B);
+  return !((K & 7) || (lda & 7) || (ldb & 7) || (at & 15)) && vb_gemm_skinny_rows(M, N, K);
 }
 
 extern "C" int vb_gemm_skinny(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, long long lda,

@@ -1197,6 +1197,7 @@ static int max_active_clusters(int bn, int cluster) {
 using namespace vb;
 
 // gemm_skinny.cu
+bool vb_gemm_skinny_rows(int M, int N, int K);
 bool vb_gemm_skinny_ok(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb);
 extern "C" int vb_gemm_skinny(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, long long lda,
                               long long ldb, long long ldc, int out_fp32, cudaStream_t stream);
@@ -1378,12 +1379,14 @@ extern "C" int vb_gemm_bf16_ws(const void* A, const void* B, void* C, const void
 
 // Gated product C [M, I] = silu(A . W[:I]^T) * (A . W[I:]^T), W = [2 I, K] = gate | up, bf16 (both factors rounded to bf16, as swiglu
 // of a product finds them). vb_gemm_swiglu_ok: 1 few rows (gemm_skinny.cu), 2 CTA pairs, 0 neither: a product and an activation.
-// Pairs under the rule of the plain product; up to 16 rows because a decode step's chain is shorter by a launch then.
+// Each under the rule of the plain product [2 I, K], whose sums the kernel takes in the same order: the result is the same bits, so a
+// pass without gradients agrees with the recorded one. (16 rows of 3584 -> 2 x 18944, which the plain product leaves to tcgen05, take 59 us
+// with an activation of their own, as before there was a gated kernel; few rows would be 54.)
 int vb_gemm_skinny_swiglu(const void* A, const void* W, void* C, int M, int I, int K, long long lda, long long ldw, long long ldc,
                           cudaStream_t stream);
 extern "C" int vb_gemm_swiglu_ok(int M, int I, int K) {
   if (M <= 0 || I <= 0 || K <= 0 || (I & 7) || (K & 7)) return 0;
-  if (M <= 16) return 1;
+  if (M <= 16 && vb_gemm_skinny_rows(M, 2 * I, K)) return 1;
   return pair_enabled() && M >= 512 && I >= 256 && K >= 256 &&
          (long long)((M + 255) / 256) * ((2ll * I + 255) / 256) >= vb_num_sms() ? 2 : 0;
 }
