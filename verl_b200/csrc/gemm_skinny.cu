@@ -126,11 +126,21 @@ using namespace vb;
 //   896 -> 9728    5.6 / 6.2 / 8.0 / 9.1 (14.6, 12.7)    2048 -> 5120   5.2 / 7.2 / 8.1 / 9.3 (13.5)
 //   3584 -> 37888  45 / 59 / 67 / 81 (66 / 52 / 46 / 46)  18944 -> 3584  23 / 27 / 32 / 40 (30 to 38)
 // Beyond 8 rows the loads of A (from L2, by every block) grow to those of B: where tiles of the tcgen05 kernel fill all SMs it is as
-// fast at 16 rows and faster beyond, and with long rows (K) its staged operands win from 24 and 32 rows on.
+// fast at 16 rows and faster beyond, and with long rows (K) its staged operands win, the earlier the fewer SMs the blocks of 16 columns
+// occupy. `most`: the longest K by rows (8, 16, 24, 32) and by N: fewer blocks than SMs, at most two blocks per SM, a second turn of the
+// SMs that is nearly empty, more. us here (tcgen05), inside | outside, matrices from memory:
+//    8 rows  768: 18944 16.8 (16.1) | 1792: 28672 25.9 (24.0)     5120: 14336 29.7 (32.1) | 18944 43.1 (39.8)    8192: 28672 72 (83)
+//   16 rows  768: 7168 9.2 (9.6) | 10240 12.4 (11.4)    2304: 14336 19.3 (19.5) | 18944 25.2 (23.1)    3584: 18944 27.0 (29.5)
+//            5120: 10240 25.0 (25.4) | 14336 34.1 (32.1)    6144: 28672 66 (78)
+//   24 rows  768: 5120 8.5 (8.4) | 6144 10.0 (9.0)    2304: 8192 15.2 (15.2)    5120: 6144 17.6 (18.4) | 4864: 8192 23.1 (21.4)
+//   32 rows  768: 3072 7.2 (7.2) | 4096 8.9 (7.8)     2304: 4096 10.5 (11.8)
 bool vb_gemm_skinny_rows(int M, int N, int K) {
-  if (M <= 8) return true;
-  if (N >= 256 * vb_num_sms()) return false;
-  return M <= 16 || (M <= 24 && K <= 8192) || (M <= 32 && K <= 4096);
+  constexpr int ANY = 0x7fffffff;
+  static const int most[4][4] = {{20480, ANY, 16384, ANY}, {8192, 16384, 10240, ANY}, {5120, 8192, 6144, 8192}, {3072, 4096, 4096, 4096}};
+  const int sms = vb_num_sms();
+  if (M > 32 || (M > 8 && N >= 256 * sms)) return false;
+  const int by_n = N < 16 * sms ? 0 : N <= 32 * sms ? 1 : N <= 40 * sms ? 2 : 3;
+  return K <= most[(M - 1) / 8][by_n] || (M <= 16 && by_n == 1 && N >= 20 * sms && K <= 20480);
 }
 bool vb_gemm_skinny_ok(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B);
