@@ -831,6 +831,25 @@ def test_routed_mlp_forms(T, E, k, H, I, first, total):
         assert err <= roundings * 2.0 ** -8 * float(want.abs().max()) + 1e-12, (got.shape, err, float(want.abs().max()))
 
 
+def test_routed_mlp_of_very_many_experts_and_pairs():
+    """Both sides of the line beyond which the places are taken by a sort, against each other."""
+    from verl_b200 import ops
+    from verl_b200.ops import moe
+
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    T, E, k, H, I = 10300, 2048, 8, 64, 64
+    x, gate_up, down = rnd(T, H).bfloat16(), rnd(E, 2 * I, H).bfloat16() * 0.1, rnd(E, H, I).bfloat16() * 0.1
+    top_i = torch.randint(0, E, (T, k), device="cuda", generator=gen)
+    top_w = torch.rand(T, k, device="cuda", generator=gen)
+    args = (gate_up, down, ops.swiglu)
+    n = 10240
+    assert moe._fused_mlp_ok(x[:n], top_i[:n], top_w[:n], *args) and not moe._fused_mlp_ok(x, top_i, top_w, *args)
+    got, want = moe.moe_mlp(x[:n], top_i[:n], top_w[:n], *args), moe.moe_mlp(x, top_i, top_w, *args)[:n]
+    # weights, terms and sums in bf16 on the general path
+    assert float((got.double() - want.double()).abs().max()) <= 4 * 2.0 ** -8 * float(want.abs().max())
+
+
 def test_routed_mlp_refuses_and_realigns():
     """Routing of another number of tokens is refused before a kernel reads past it; rows and gradients off a 16-byte boundary work."""
     from verl_b200 import ops
