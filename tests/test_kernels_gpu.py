@@ -457,6 +457,105 @@ def test_sampler_support_and_logprob(V, B, k, p):
     assert float((lp - ref).abs().max()) < 2e-5  # fast exp, log and fp32 sums of up to 40 terms
 
 
+def _sampler_bounds(logits, k, p):
+    """Of one row in fp64: log-probs, and which tokens are inside for sure and at most. The threshold is searched in fp32: probabilities
+    (fast exp, 2^-21 and the sum's error) within 1e-4 of it, and masses within 1e-5 of ``p``, may fall on either side."""
+    lp = torch.log_softmax(logits.double(), -1)
+    q = lp.exp()
+    d = q.sort(descending=True).values
+    cum = d.cumsum(0)
+
+    def threshold(mass):
+        thr = d[k - 1] if 0 < k < d.numel() else d[-1] * 0
+        return torch.maximum(thr, d[min(int((cum < mass).sum()), d.numel() - 1)]) if p < 1 else thr
+
+    at_most = q >= threshold(p + 1e-5) * (1 - 1e-4) - d[0] * 2.0 ** -29
+    return lp, q >= threshold(p - 1e-5) * (1 + 1e-4), at_most
+
+
+@pytest.mark.parametrize("V,B", [(1024, 3), (1025, 3), (4099, 3), (32771, 3), (152064, 3), (152064, 40), (32771, 150)])  # 1 to 8 blocks per row
+@pytest.mark.parametrize("kind,k,p", [("flat", -1, 0.9), ("flat", 900, 1.0), ("flat", 5000, 1.0), ("flat", 3000, 0.5), ("equal", 50, 1.0),
+                                      ("equal", -1, 0.3), ("equal", 7, 0.99), ("ties", 1000, 1.0), ("ties", -1, 0.6), ("steps", 2500, 1.0)])
+def test_sampler_wide_supports(V, B, kind, k, p):
+    """Supports above the short list (1024 tokens): guesses that narrow, counting on the row, the hand-over of what lies between the
+    bounds, and more equal probabilities at the threshold than the list holds."""
+    from verl_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(V + B)
+    logits = torch.randn(B, V, device="cuda", generator=gen)
+    if kind == "flat":
+        logits *= 0.5
+    elif kind == "equal":
+        logits[:] = 0.25
+    elif kind == "ties":  # 300 stronger ones, then 3000 equal ones (or what there is), the rest far below
+        order = torch.rand(B, V, device="cuda", generator=gen).argsort(-1)
+        value = torch.full((V,), -20.0, device="cuda")
+        value[:3300] = 1.0
+        value[:300] = 2.0 + torch.rand(300, device="cuda", generator=gen)
+        logits.scatter_(1, order, value.expand(B, V).contiguous())
+    else:  # ten levels of equal tokens
+        logits = (torch.rand(B, V, device="cuda", generator=gen) * 10).floor() * 0.3
+    tok, lp = ops.sample(logits, top_k=torch.full((B,), k, dtype=torch.int32, device="cuda"), top_p=torch.full((B,), p, device="cuda"),
+                         seed=9, step=torch.zeros(1, dtype=torch.long, device="cuda"))
+    for b in range(0, B, max(1, B // 5)):
+        full, least, most = _sampler_bounds(logits[b], k, p)
+        t = int(tok[b])
+        assert bool(most[t]), (b, t)
+        lo, hi = (float(full[t] - torch.logsumexp(full[m], 0)) for m in (most, least if bool(least.any()) else most))
+        assert lo - 5e-5 <= float(lp[b]) <= hi + 5e-5, (b, lo, float(lp[b]), hi)  # fast exp and log, fp32 sums of up to V terms
+
+
+@pytest.mark.parametrize("V", [1000, 5000, 152064])
+def test_sampler_rows_without_numbers(V):
+    """Rows of NaN, of -inf, with some of either, and with +inf: a token of the vocabulary comes out, a masked one never, and the other
+    rows are as they are without them."""
+    from verl_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(V)
+    x = torch.randn(7, V, device="cuda", generator=gen) * 3
+    clean = x.clone()
+    x[0] = float("nan")
+    x[1, 17] = float("nan")
+    x[2] = float("-inf")
+    x[4, 33] = float("inf")
+    for rows in (x, clean):
+        rows[3, ::2] = float("-inf")
+        rows[6, : V - 3] = float("-inf")
+    for k, p, t in ((-1, 1.0, 1.0), (-1, 1.0, 0.0), (50, 1.0, 1.0), (-1, 0.9, 0.7), (20, 0.8, 1.0), (900, 1.0, 1.3)):
+        outs = []
+        for rows in (x, clean):
+            full = lambda v, dt: torch.full((7,), v, dtype=dt, device="cuda")  # noqa: E731
+            outs.append(ops.sample(rows, temperature=full(t, torch.float32), top_k=full(k, torch.int32), top_p=full(p, torch.float32),
+                                   seed=5, step=torch.zeros(1, dtype=torch.long, device="cuda")))
+        (tok, lp), (tok_c, lp_c) = outs
+        assert bool(((tok >= 0) & (tok < V)).all())
+        for r in (3, 5, 6):
+            assert int(tok[r]) == int(tok_c[r]) and float(lp[r]) == float(lp_c[r])
+        assert int(tok[3]) % 2 == 1 and int(tok[6]) >= V - 3
+
+
+@pytest.mark.parametrize("B", [3, 30, 75])
+def test_sampler_mixed_rows(B):
+    """Restricted, free and greedy rows in one call give the bits that each gives among rows of its own kind."""
+    from verl_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(B)
+    logits = torch.randn(B, 32771, device="cuda", generator=gen) * 2
+    kinds = [(1.0, -1, 1.0), (0.0, 50, 0.9), (0.8, 40, 1.0), (1.0, -1, 0.95), (0.7, 2000, 0.99)]  # temperature, top-k, top-p
+
+    def call(of):
+        cols = list(zip(*(kinds[i] for i in of)))
+        return ops.sample(logits, temperature=torch.tensor(cols[0], device="cuda"), top_k=torch.tensor(cols[1], dtype=torch.int32, device="cuda"),
+                          top_p=torch.tensor(cols[2], device="cuda"), seed=1, step=torch.zeros(1, dtype=torch.long, device="cuda"))
+
+    of = [b % len(kinds) for b in range(B)]
+    tok, lp = call(of)
+    for i in range(len(kinds)):
+        t, l = call([i] * B)
+        rows = torch.tensor([o == i for o in of], device="cuda")
+        assert torch.equal(t[rows], tok[rows]) and torch.equal(l[rows], lp[rows])
+
+
 def test_sampler_never_takes_a_token_of_no_weight():
     """A uniform draw that rounds up to one must not become infinite noise: 4000 rows of 152 064 tokens hold about 36 such draws."""
     from verl_b200 import ops
