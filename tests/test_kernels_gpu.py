@@ -675,8 +675,7 @@ def test_qkv_heads_gradients(T, Hq, Hk, D, norm):
                                                  (4, 40, 8, 128, 16, 150), (3, 32, 2, 128, 128, 1000),
                                                  (2, 8, 8, 128, 8, 260), (1, 14, 2, 64, 16, 110), (7, 8, 8, 64, 8, 129),
                                                  (3, 32, 2, 64, 32, 1025), (40, 8, 1, 64, 256, 2100), (3, 9, 1, 128, 16, 513),
-                                                 # more (sequence, head, split) items than resident CTAs: the
-                                                 # persistent kernel (CTAs walk several items, some of them empty)
+                                                 # more (sequence, head, split) CTAs than run at once, some of them without keys
                                                  (100, 28, 4, 128, 16, 700), (80, 32, 8, 128, 16, 300)])
 def test_paged_decode_attention(B, Hq, Hk, D, bs, maxlen):
     from verl_b200 import ops
@@ -752,6 +751,41 @@ def test_decode_attention_weights_stay_in_fp32(Hq, Hk, D, bs, lens):
         want = torch.einsum("hgk,hkd->hgd", p, v).reshape(Hq, D)
         # scores of up to about 5 in fp32 and sums of L weights: 2^-24 each, some tens of them together; weights in bf16 would be 2^-10 off
         assert float((got[b] - want).norm() / want.norm()) <= 64 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("sigmoid", [False, True])
+@pytest.mark.parametrize("B,Hq,Hk,D,splits,window", [(160, 8, 2, 128, 1, 0), (120, 8, 2, 64, 3, 150), (75, 40, 8, 96, 2, 0), (310, 3, 1, 128, 4, 70)])
+def test_windowed_decode_walks_several_items_per_cta(B, Hq, Hk, D, splits, window, sigmoid):
+    """More (sequence, KV head, split) items than CTAs run at once: the tcgen05 kernel of the layer-list models takes one after the
+    other, with items in between that have no key (short sequences, windows), and none may see what the one before left."""
+    from verl_b200 import ops
+    from verl_b200.ops import _lib
+
+    gen = torch.Generator().manual_seed(B + splits)
+    bs, most = 16, 700
+    assert B * Hk * splits > 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    lens = torch.randint(1, most, (B,), generator=gen, dtype=torch.int32)
+    lens[::7] = torch.randint(1, 40, (len(lens[::7]),), generator=gen, dtype=torch.int32)
+    n = (most + bs - 1) // bs
+    q, kc, vc = (torch.randn(*s, generator=gen).bfloat16() for s in ((B, Hq, D), (B * n, Hk, bs, D), (B * n, Hk, bs, D)))
+    table = torch.randperm(B * n, generator=gen).int().reshape(B, n)
+    scale, opts = D ** -0.5, dict(window=window)
+    shift = r1 = r2 = None
+    if sigmoid:
+        shift, r1, r2 = torch.randn(Hq, generator=gen) - 3, torch.rand(Hq, generator=gen) * 0.3, torch.rand(Hq, generator=gen) * 0.1
+        opts.update(shift=shift, log_bias=(r1, r2))
+    cu = torch.arange(B + 1, dtype=torch.int32)
+    ref = ops.paged_attention(q.float(), kc.float(), vc.float(), table, cu, lens, 1, scale=scale, **opts)
+    q, kc, vc, table, lens_d = (t.cuda() for t in (q, kc, vc, table, lens))
+    shift, r1, r2 = (None if t is None else t.cuda() for t in (shift, r1, r2))
+    work = torch.full((B * Hq * splits * (D + 2),), float("nan"), device="cuda")
+    out = torch.full((B, Hq * D), float("nan"), dtype=torch.bfloat16, device="cuda")
+    rc = _lib.fn("vb_paged_decode_window")(q.data_ptr(), q.stride(0), kc.data_ptr(), vc.data_ptr(), kc.shape[0], table.data_ptr(),
+                                           table.stride(0), lens_d.data_ptr(), B, Hq, Hk, D, D, bs, scale, window, 0, 0, None, 0, 0.0, None,
+                                           _lib.ptr(shift), _lib.ptr(r1), _lib.ptr(r2), None, 0, 0, splits, out.data_ptr(), out.stride(0),
+                                           work.data_ptr() if splits > 1 else None, _lib.status_word("cuda").data_ptr(), _lib.stream())
+    assert rc == 0 and _lib.read_status("cuda")[0] == 0
+    _bf16_close(out, ref, ulps=4)
 
 
 def _attn_ref(q, k, v, cu, causal, scale):
@@ -1293,3 +1327,53 @@ def test_kernels_write_inside_their_buffers():
         ops.lmhead_logprob_entropy(h, wl, torch.randint(0, 1000, (100,), device=dev), 1.0)
         n_checked = g.check()
     assert n_checked >= 30
+
+
+def test_fused_kernels_write_inside_their_buffers():
+    """The same for the few-row and fp8 decode products, gated units, head norms with positions, routed experts, column sums, decode
+    attention of heads of 64 and restricted sampling, forward and backward, on ragged sizes."""
+    from verl_b200 import ops
+    from verl_b200.ops import fp8
+    from verl_b200.ops.gemm import colsum
+    from verl_b200.ops.moe import moe_gate, moe_mlp
+    from verl_b200.utils.debug.guard_bands import guard_allocations
+
+    torch.manual_seed(6)
+    dev = "cuda"
+    rnd = lambda *s: torch.randn(*s, device=dev).bfloat16()  # noqa: E731
+    with guard_allocations() as g:
+        with torch.no_grad():
+            for M in (1, 9, 17, 31):
+                ops.gemm(rnd(M, 520), rnd(1153, 520))
+                ops.gemm(rnd(M, 72), rnd(33, 72), out_dtype=torch.float32)
+            for M, I, K in ((3, 24, 72), (16, 296, 136), (601, 4872, 264)):
+                ops.linear_swiglu(rnd(M, K), rnd(2 * I, K))
+            for M, N, K in ((1, 136, 144), (33, 200, 1040), (65, 520, 3584)):
+                wq, sw = fp8.quantize_weight(rnd(N, K))
+                fp8.fp8_linear(rnd(M, K), wq, sw, None)
+        for T, Hq, Hk, D in ((1, 14, 2, 64), (37, 5, 1, 128), (3, 2, 2, 256)):
+            pos, tables = torch.arange(T, device=dev), ops.rope_tables(D, 512, 10000.0, dev)
+            for norms in (None, (rnd(D).requires_grad_(True), rnd(D).requires_grad_(True))):
+                qkv = rnd(T, (Hq + 2 * Hk) * D).requires_grad_(True)
+                heads = ops.qkv_heads(qkv, pos, *tables, Hq, Hk, D, norms, 1e-6)
+                torch.autograd.backward(heads, [torch.randn_like(h) for h in heads])
+                with torch.no_grad():
+                    ops.qkv_heads(qkv, pos, *tables, Hq, Hk, D, norms, 1e-6, in_place=False)
+        for T, E, k, H, I in ((1, 8, 2, 64, 64), (45, 33, 8, 192, 64), (300, 4, 1, 128, 128)):
+            z = rnd(T, E).requires_grad_(True)
+            w, idx = moe_gate(z, k, True)
+            leaves = [t.requires_grad_(True) for t in (rnd(T, H), rnd(E, 2 * I, H), rnd(E, H, I))]
+            moe_mlp(leaves[0], idx, w, leaves[1], leaves[2], ops.swiglu).backward(rnd(T, H))
+        for T, N in ((7, 34), (513, 1026)):
+            colsum(rnd(T, N))
+        B, Hq, Hk, D, bs, ctx = 5, 14, 2, 64, 16, 77
+        n = (ctx + bs - 1) // bs
+        table = torch.arange(B * n, device=dev, dtype=torch.int32).reshape(B, n)
+        lens = torch.tensor([ctx, 1, 16, 17, 64], device=dev, dtype=torch.int32)
+        for splits in (1, 3):
+            ops.paged_decode_attention(rnd(B, Hq, D), rnd(B * n, Hk, bs, D), rnd(B * n, Hk, bs, D), table, lens, num_splits=splits)
+        for rows, V in ((3, 5003), (150, 1025)):
+            full = lambda v, dt: torch.full((rows,), v, dtype=dt, device=dev)  # noqa: B023,E731
+            ops.sample(torch.randn(rows, V, device=dev), top_k=full(20, torch.int32), top_p=full(0.9, torch.float32), seed=3)
+        n_checked = g.check()
+    assert n_checked >= 60
