@@ -17,11 +17,6 @@ __device__ __forceinline__ uint4 ld_stream(const __nv_bfloat16* p) {
   asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 constexpr int SK_WARPS = 8;
 
@@ -78,8 +73,8 @@ gemm_skinny_kernel(const __nv_bfloat16* A, const __nv_bfloat16* B, void* __restr
 #pragma unroll
           for (int j = 0; j < NT; ++j) {
             const uint4 lo = w[u][h][2 * r], hi = w[u][h][2 * r + 1], v = x[u][h][j];
-            mma_16816(acc[r][j], lo.x, hi.x, lo.y, hi.y, v.x, v.y);
-            mma_16816(acc[r][j], lo.z, hi.z, lo.w, hi.w, v.z, v.w);
+            mma_bf16(acc[r][j], lo.x, hi.x, lo.y, hi.y, v.x, v.y);
+            mma_bf16(acc[r][j], lo.z, hi.z, lo.w, hi.w, v.z, v.w);
           }
   }
 #pragma unroll

@@ -167,7 +167,8 @@ def paged_decode_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torc
     seq_lens int32 [B] (including the current token, already written to the cache).
 
     ``impl``: "tc" = tensor-core kernel (head_dim 128, <= 16 query heads per KV head, block size a power of two in
-    8..128), "simt" = CUDA-core kernel, "auto" = the tensor-core kernel wherever it applies."""
+    8..128: softmax weights in bf16), "simt" = CUDA-core kernel (weights in fp32), "auto" = the tensor-core kernel wherever it
+    applies, which takes heads of 64 and larger blocks too, with weights in fp32."""
     B, Hq, D = q.shape
     Hk, BS = k_cache.shape[1], k_cache.shape[2]
     scale = scale if scale is not None else D ** -0.5

@@ -273,7 +273,7 @@ def _bench_attention(add, r, att, ref, B: int, n: int, DB: int, ctx: int) -> Non
     add(f"paged_decode_window ({what}: {seen} keys)", time_us(lambda: ops.paged_attention(
         q1, kc, vc, bt, cu1, lens, 1, max_ctx=ctx, **kw_, gate=gate[:DB] if att.gate else None)), DB * seen * hk * d * 4)
     splits, work = ops.decode_workspace(DB, hq, hk, d, ctx, "cuda")
-    add("  vs paged_decode_tc (full context)", time_us(
+    add("  vs paged_decode_attention (full context)", time_us(
         lambda: ops.paged_decode_attention(q1, kc, vc, bt, lens, num_splits=splits, work=work)), DB * ctx * hk * d * 4)
 
 
