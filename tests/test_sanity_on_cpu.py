@@ -102,3 +102,31 @@ def test_short_cuts_are_off_where_something_follows_the_computation():
             seen.append((_lib.plain(), _lib.followed()))
         assert _lib.plain()
     assert seen == [(False, True), (False, True)]
+
+
+def test_threads_share_one_word_for_refused_indices(monkeypatch):
+    """Kernels keep its address: a second one made at the same time would leave the first to the allocator's next user."""
+    import threading
+    import time
+
+    import torch
+
+    from verl_b200.ops import _lib
+
+    made = []
+
+    def slow_zeros(*size, dtype, pin_memory, _zeros=torch.zeros):
+        time.sleep(0.05)
+        made.append(_zeros(*size, dtype=dtype))
+        return made[-1]
+
+    monkeypatch.setattr(_lib, "_refused", None)
+    monkeypatch.setattr(torch, "zeros", slow_zeros)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    got = []
+    threads = [threading.Thread(target=lambda: got.append(_lib.refused_word())) for _ in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(made) == 1 and got == [made[0].data_ptr()] * 8

@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from ctypes import c_float, c_int, c_longlong, c_ulonglong, c_void_p
 from pathlib import Path
 
@@ -253,6 +254,7 @@ def clear_status(device=None) -> None:
 
 
 _refused = None
+_refused_lock = threading.Lock()
 
 
 def refused_word() -> int | None:
@@ -262,8 +264,10 @@ def refused_word() -> int | None:
     if _refused is None:
         if torch.cuda.is_current_stream_capturing():
             return None
-        words = torch.zeros(4, dtype=torch.int32, pin_memory=True)
-        _refused = words, (c_int * 4).from_address(words.data_ptr())
+        with _refused_lock:  # one for the process: kernels keep the address
+            if _refused is None:
+                words = torch.zeros(4, dtype=torch.int32, pin_memory=True)
+                _refused = words, (c_int * 4).from_address(words.data_ptr())
     return _refused[0].data_ptr()
 
 
