@@ -75,3 +75,46 @@ def test_second_backward_recomputes_a_kept_unit():
         once = eng.zero.grad.clone()
         loss.backward()
     torch.testing.assert_close(eng.zero.grad, 2 * once)
+
+
+def test_forwards_that_wait_for_their_backward_count_in_what_is_kept(monkeypatch):
+    """Small micro-batches are kept without a look at the memory, but only one at a time: with several forwards before a backward the
+    next one asks what is free."""
+    import torch
+
+    from verl_b200.models import preset
+    from verl_b200.models.transformer import PackedBatch
+    from verl_b200.workers.engine.native import NativeEngine
+
+    cfg = preset("tiny-qwen2")
+    ids = torch.randint(3, cfg.vocab_size, (20,), generator=torch.Generator().manual_seed(0))
+    batch = PackedBatch(ids, torch.arange(20), torch.tensor([0, 20], dtype=torch.int32), 20)
+    eng = NativeEngine(cfg, {}, {"lr": 1e-3}, device="cpu", seed=1).initialize()
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (1 << 30, 180 << 30))
+    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda device=None: 0)
+    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda device=None: 0)
+
+    def layers_kept():  # as the engine decides on a GPU with 1 GB left
+        monkeypatch.setattr(eng, "device", torch.device("cuda", 0))
+        n = eng._layers_to_keep(20)
+        monkeypatch.setattr(eng, "device", torch.device("cpu"))
+        return n
+
+    def forward():
+        return -eng.forward_logprob(batch, torch.arange(19), ids[1:], 1.0)[0].mean()
+
+    with eng.train_mode():
+        monkeypatch.setattr(eng, "engine_config", {"keep_activation_layers": cfg.num_hidden_layers})
+        eng.optimizer_zero_grad()
+        losses = [forward()]
+        monkeypatch.setattr(eng, "engine_config", {})
+        assert layers_kept() == 0
+        losses.append(forward())
+        losses[0].backward()
+        assert layers_kept() == 0  # the second one's head still waits
+        losses[1].backward()
+        assert layers_kept() == cfg.num_hidden_layers
+        forward()  # nobody goes back through it
+        assert layers_kept() == 0
+        eng.optimizer_zero_grad()
+        assert layers_kept() == cfg.num_hidden_layers

@@ -72,6 +72,7 @@ class ZeroShardedParams:
         self.comm = comm  # optional accelerated collectives (peer-memory kernels); falls back to torch.distributed
         self.units: list[ZeroUnit] = []
         self._anchor = None
+        self.kept_waiting = 0  # unit calls since zero_grad that keep activations for a backward still to come
         seen: set[int] = set()
         off = 0
         for spec in units:
@@ -323,6 +324,7 @@ class ZeroShardedParams:
         return missing
 
     def zero_grad(self):
+        self.kept_waiting = 0
         if self.trainable:
             self.wait_comm()
             self.grad.zero_()
@@ -442,6 +444,7 @@ class _UnitFnKeep(torch.autograd.Function):
             zero.release(unit)
         ctx.single = not isinstance(outs, tuple)
         ctx.inputs, ctx.outs = inputs, ((outs,) if ctx.single else outs)
+        zero.kept_waiting += 1
         det = tuple(o.detach() if isinstance(o, torch.Tensor) else o for o in ctx.outs)
         return det[0] if ctx.single else det
 
@@ -452,6 +455,7 @@ class _UnitFnKeep(torch.autograd.Function):
         zero, unit = ctx.zero, ctx.unit
         inputs, outs = ctx.inputs, ctx.outs
         ctx.inputs = ctx.outs = None
+        zero.kept_waiting = max(0, zero.kept_waiting - 1)
         zero.gather(unit, for_backward=True)
         try:
             pairs = [(o, g) for o, g in zip(outs, grads) if g is not None and isinstance(o, torch.Tensor) and o.requires_grad]

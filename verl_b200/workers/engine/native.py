@@ -632,7 +632,9 @@ class NativeEngine(BaseEngine):
         else:
             inner = tokens * 6 * c.intermediate_size
         per_layer = int((tokens * per_token + inner) * 1.1)
-        if n_layers * per_layer <= 1 << 28:  # 256 MB: kept without asking what is free, which takes 1.6 ms of a small micro-batch's 10
+        # 256 MB are kept without asking what is free, which takes 1.6 ms of a small micro-batch's 10; not on top of what earlier forwards
+        # keep for a backward that is still to come (a pipeline's micro-batches, a sum of losses): together they could be any amount
+        if n_layers * per_layer <= 1 << 28 and self.zero.kept_waiting == 0:
             self.last_kept_layers = n_layers
             return n_layers
         free, total = torch.cuda.mem_get_info(self.device)
